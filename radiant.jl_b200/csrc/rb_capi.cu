@@ -763,9 +763,7 @@ static LaunchShape choose_shape(const std::vector<const DevProblem *> &hs, int c
     const long long gsz = (long long)sizeof(rb::GroupShared);
     const long long b1 = (std::min<long long>(optin, (long long)per_sm - reserved) - gsz) & ~15LL;
     LaunchShape sh{cluster, 0, (size_t)gsz};
-    bool any = false;  // some problem takes the local 1D pass or the 3D octant sweep
-    for (const DevProblem *h : hs) any = any || rb::local1d_ok(*h, 1 << 4, 1LL << 40) || h->ndims == 3;
-    if (!any || b1 <= 0) return sh;
+    if (hs.empty() || b1 <= 0) return sh;
     auto fits = [&](int C, bool w) {  // every local-shaped 1D problem fits the local pass at cluster C
         for (const DevProblem *h : hs)
             if (rb::local1d_ok(*h, C, 1LL << 40) && !(w ? rb::local1d_w(*h, C, b1) : rb::local1d_ok(*h, C, b1)))
@@ -846,8 +844,9 @@ int launch_grid(rb_context *ctx, DevProblem *prob, const DevProblem &hp, cudaStr
     const bool mixed = h.precision == 1;
     long long need = 0;
     if (h.ndims == 3 && h.nm5 == 1 && h.nm4 == 1 && h.nmf[0] == 1 && h.nmf[1] == 1 && h.nmf[2] == 1)
-        need = mixed ? (h.csd ? rb::oct3d_smem<float, true>() : rb::oct3d_smem<float, false>())
-                     : (h.csd ? rb::oct3d_smem<double, true>() : rb::oct3d_smem<double, false>());
+        need = std::max(rb::oct3d_smem<float>(h.csd), rb::oct3d_smem<double>(h.csd));
+    if (h.ndims == 2)
+        need = h.nm5 == 1 ? std::max(rb::sweep2d_bytes(h.nx, 0, h.csd), rb::sweep2d_bytes(h.nx, 1, h.csd)) : rb::sweep2d_hi_bytes(h);
     if (mixed && h.tc_m2d) {  // the products: operator resident where it fits, else streamed
         const int parts = h.mnfp ? 2 : 1;
         auto plan = [&](int nj, int nk) {
@@ -855,6 +854,16 @@ int launch_grid(rb_context *ctx, DevProblem *prob, const DevProblem &hp, cudaStr
             return r <= avail ? r : rb::tc::bytes_streamed(rb::tc::round16(nj));
         };
         need = std::max(need, std::max(plan(h.nd, parts * h.np), plan(h.np, h.nd)));
+    }
+    if (!mixed || h.nm5 > 1) {  // the FP64 products: whole operators where they fit, else in row blocks
+        const int parts = h.mnfp ? 2 : 1;
+        auto plan = [&](int ni, int nk, int p) {
+            const int nrb = rb::prod_blocks(ni, nk, p, avail);
+            if (nrb == 0) return avail;
+            const int tiles = (ni + 7) / 8;
+            return rb::prod_bytes(rb::prod_nt(8 * ((tiles + nrb - 1) / nrb)), nk, p);
+        };
+        need = std::max(need, std::max(plan(h.nd, h.np, parts), plan(h.np, h.nd, 1)));
     }
     if (need > avail) need = 0;  // the problem then takes the paths that need no region
     const int local_bytes = (int)((need + 1023) & ~1023LL);
@@ -865,7 +874,7 @@ int launch_grid(rb_context *ctx, DevProblem *prob, const DevProblem &hp, cudaStr
     if (per_sm < 1) return fail(ctx, RB_ERR_CUDA, "the grid solve kernel does not fit on an SM");
     if (per_sm > 1) per_sm = 1;
     const int grid = ctx->nsm * per_sm;
-    if (!ctx->d_gpart) CK(cudaMalloc(&ctx->d_gpart, sizeof(double) * 2 * 4 * 4096));
+    if (!ctx->d_gpart) CK(cudaMalloc(&ctx->d_gpart, sizeof(double) * ((size_t)8 * grid * grid + 2 * (size_t)RB_SM * grid)));
     void *args[] = {(void *)&prob, (void *)&ctx->d_gpart, (void *)&local_bytes};
     CK(cudaLaunchCooperativeKernel((void *)rb::solve_grid_kernel, dim3(grid), dim3(RB_THREADS), args, smem, s));
     return RB_OK;
@@ -962,6 +971,27 @@ ProblemRec *find(rb_context *ctx, rb_handle h) {
     return it == ctx->probs.end() ? nullptr : it->second.get();
 }
 
+// Whether the FP64 passes of a mixed 3D one-moment problem on the whole GPU solve a cell as
+// sweep_3d_tiles does (products with h = |Ω|/Δ, the reciprocal of the collision term) instead of as
+// the octant sweep: the form those passes have had for the problems without CSD whose operators'
+// shared memory left no room for the octant sweep's FP64 stages (128 208 bytes). The FP32 passes
+// between them follow the last bit of these passes (BiCGStab carries it to 1e-8 of the flux), so the
+// form is part of the mixed result and stays.
+static int mixed_recip(const DevProblem &h, bool tc) {
+    if (h.precision != 1 || h.ndims != 3 || h.nm5 != 1 || h.csd) return 0;
+    const long long avail = 183296;
+    long long need = 83888;
+    if (tc) {
+        auto plan = [&](int nj, int nk) {
+            const long long r = rb::tc::bytes_resident(rb::tc::round16(nj), nk);
+            return r <= avail ? r : rb::tc::bytes_streamed(rb::tc::round16(nj));
+        };
+        need = std::max(need, std::max(plan(h.nd, h.np), plan(h.np, h.nd)));
+    }
+    if (need > avail) need = 0;
+    return ((need + 1023) & ~1023LL) < 128208;
+}
+
 // Lays one problem out in the device block `b` (offsets `o` from required()): fills the
 // device record `h`, queues the table copies on `s` and writes the record to *dptr.
 // Source definitions of rb_upload_sources and where their device copies sit in the block.
@@ -990,6 +1020,10 @@ int place_problem(rb_context *ctx, const rb_sn_problem *P, const Derived &D, con
     h.vstride = (D.nstate + 1) & ~1LL;
     for (int a = 0; a < 4; a++) h.w1[a] = D.w1[a];
     for (int f = 0; f < 6; f++) h.bc[f] = P->bc[f];
+    h.psi_sn = P->ndims == 2 ? (long long)nm5 * D.ncell : 1;
+    h.psi_sc = P->ndims == 2 ? 1 : nd;
+    h.pe_sn = P->ndims == 2 ? (long long)h.nm4 * D.ncell : 1;
+    h.recip = mixed_recip(h, !D.tc_m2d.empty());
     h.noct = D.noct;
     for (int o = 0; o <= 8; o++) h.oct_start[o] = D.oct_start[o];
 #define DP(T, k) (reinterpret_cast<T *>(b + o[k]))

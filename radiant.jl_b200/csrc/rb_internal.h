@@ -33,11 +33,16 @@ struct DevProblem {
     int np_source;
     long long nphi, nstate, off_b[3], nb[3];
     long long fcells[3];  // boundary face cells per axis
+    int recip;         // mixed 3D form: the FP64 passes solve a cell by the reciprocal (rb_capi.cu)
     int noct;          // direction groups: 1 (1D), 4 quadrants (2D), 8 octants (3D)
     int oct_start[9];  // device directions of group o: [oct_start[o], oct_start[o+1]); 2D/3D
                        // problems hold their directions sorted by group (bit 0: μ < 0,
                        // bit 1: η < 0, bit 2: ξ < 0), the reference's order inside a group
     int nvec;          // Krylov vectors allocated in `vecs`
+    // angular arrays (ψ, Mn·Qlout, energy-face fluxes) hold direction n of column col (a cell's moment)
+    // at n·psi_sn + col·psi_sc: directions fastest (1, nd), or, in 2D, whose sweeps walk the cells of
+    // one direction, columns fastest (nm5·ncell, 1); pe_sn is psi_sn of the energy-face fluxes
+    long long psi_sn, psi_sc, pe_sn;
     long long vstride; // distance between Krylov vectors: nstate rounded up to even (the pad stays 0)
     // ---- tables (device pointers) --------------------------------------------------------
     const double *dx, *dy, *dz;

@@ -11,7 +11,8 @@ __global__ void __launch_bounds__(RB_THREADS, 1) solve_grid_kernel(DevProblem *p
     GroupShared &gs = *reinterpret_cast<GroupShared *>(smem_raw);
     void *local = local_bytes > 0 ? (void *)(smem_raw + sizeof(GroupShared)) : nullptr;
     GridTeam t;
-    t.init(&gs.team, gpart);
+    t.init(&gs.team, gpart, gs.tile);
+    t.ordered = prob->precision == 1;
     // the mixed form's 2D/3D products run on the tensor cores: every CTA holds TMEM columns for
     // their accumulators and the mbarriers of MMA completion for the whole launch
     const bool use_tc = prob->precision == 1 && prob->ndims >= 2 && prob->tc_m2d != nullptr;

@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include "rb_internal.h"
+#include "rb_product.cuh"
 #include "rb_team.cuh"
 
 #define RB_MAXRESTART 48
@@ -249,9 +250,14 @@ struct alignas(16) GroupShared {
         };
         // M2D / D2M: a tile of columns of the moment or angular arrays
         double tile[RB_TILE_DOUBLES];
+        // Gram-Schmidt: the reductions' scratch
+        double red[RB_SM_DOUBLES];
     };
     TeamShared team;
     TcState tc;
+    DevProblem prob;    // the problem in work (its fields are read in every phase; a team barrier drops
+                        // them from L1, so each read from the global record cost an L2 round trip)
+    alignas(16) unsigned char l1d[256];  // Local1D of the problem in work (rb_local1d.cuh)
     unsigned oct_epoch;  // 3D octant sweeps run so far in this solve (identical in every CTA)
 };
 
@@ -403,7 +409,7 @@ struct Cell1D {
                 R a = w1E * FE[e];
 #pragma unroll
                 for (int j = 0; j < NM; j++) a += (R)P.Eout[e + NE * j] * q[0][j];
-                phiE_out[n + (long long)nd * (e + (long long)NE * c)] = (double)a;
+                if (phiE_out) phiE_out[n + (long long)nd * (e + (long long)NE * c)] = (double)a;
             }
         }
         PS *pc = psi + n + ld * NM * (c - c0);
@@ -573,7 +579,7 @@ static __device__ void sweep1d_dir_rt(const DevProblem &P, const GroupShared &gs
                 double a = P.w1[3] * FE[e];
 #pragma unroll 1
                 for (int j = 0; j < nm; j++) a += P.Eout[e + ne * j] * q[j];
-                phiE_out[n + (long long)nd * (e + (long long)ne * c)] = a;
+                if (phiE_out) phiE_out[n + (long long)nd * (e + (long long)ne * c)] = a;
             }
         }
 #pragma unroll 1
@@ -637,8 +643,8 @@ template <class TX>
 struct ProductArgs {
     const double *A, *B;   // [ni + lda·k] operators (B may be null)
     int lda, ni, nk;
-    const TX *X;           // [k + ldx·col]
-    int ldx;
+    const TX *X;           // [k·sx + ldx·col]
+    long long sx, ldx;
     long long ncol;
 };
 
@@ -714,7 +720,7 @@ __device__ void team_product(Team &t, GroupShared &gs, const ProductArgs<TX> &a,
                 const int k = k0 + e % KC;
                 const long long col = c0 + e / KC;
                 const bool in = e < KC * TC && k < kend && col < a.ncol;
-                xv[u] = in ? (double)a.X[(k < nk ? k : k - nk) + (long long)a.ldx * col] : 0.0;
+                xv[u] = in ? (double)a.X[(k < nk ? k : k - nk) * a.sx + a.ldx * col] : 0.0;
                 sv[u] = in ? scale(k, col) : 0.0;
             }
             __syncthreads();
@@ -777,50 +783,54 @@ __device__ void team_product(Team &t, GroupShared &gs, const ProductArgs<TX> &a,
 }
 
 // ψ[n,col] = add[n,col] + Σ_p Mn[n,p]·ys[mat,p]·𝚽[p,col] + Σ_p (Mn·ℳ)[n,p]·T[mat]·𝚽[p,col]
-// (scaled == 0: ψ = Mn·src, the Mn·Qlout product of the group set-up). The mixed form computes
-// it in FP32 into the FP32 angular buffer (the FP64 Mn·Qlout term is added before rounding).
+// (scaled == 0: out = Mn·src, the Mn·Qlout product of the group set-up) into `out` in FP64. The
+// mixed form computes it in FP32 into the FP32 angular buffer (the FP64 Mn·Qlout term is added
+// before rounding).
 template <class Team>
-__device__ void m2d_tiles(Team &t, const DevProblem &P, GroupShared &gs, const double *src, const double *add,
-                          int scaled, int mixed = 0) {
+__device__ void m2d_tiles(Team &t, const DevProblem &P, GroupShared &gs, void *region, long long bytes,
+                          const double *src, const double *add, double *out, int scaled, int mixed = 0) {
     const int nd = P.nd, np = P.np, nm = P.nm5;
-    ProductArgs<double> a{P.mn, (scaled && P.mnfp) ? P.mnfp : nullptr, nd, nd, np, src, np, (long long)nm * P.ncell};
+    const long long ncol = (long long)nm * P.ncell, sn = P.psi_sn, sc_ = P.psi_sc;
     const int *mat = P.mat;
     const double *ys = P.kmat;
-    auto sc = [=, &gs] __device__(int k, long long col) {
-        if (!scaled) return 1.0;
-        const int m = mat[col / nm];
-        return k < np ? ys[(long long)m * np + k] : gs.tg[m];
-    };
-    auto pre = [=] __device__(int i, long long col) { return add ? add[col * nd + i] : 0.0; };
     if (mixed && scaled) {
+        ProductArgs<double> a{P.mn, P.mnfp, nd, nd, np, src, 1, np, ncol};
+        auto sc = [=, &gs] __device__(int k, long long col) {
+            const int m = mat[col / nm];
+            return k < np ? ys[(long long)m * np + k] : gs.tg[m];
+        };
+        auto pre = [=] __device__(int i, long long col) { return add ? add[col * sc_ + i * sn] : 0.0; };
         float *psi = P.psi32;
         team_product<float>(t, gs, a, sc, pre, [=] __device__(int i, long long col, double v, double ad) {
-            psi[col * nd + i] = (float)(ad + v);
+            psi[col * sc_ + i * sn] = (float)(ad + v);
         });
         return;
     }
-    double *psi = P.psi;
-    team_product<double>(t, gs, a, sc, pre, [=] __device__(int i, long long col, double v, double ad) {
-        psi[col * nd + i] = ad + v;
-    });
+    Prod64 a{P.mn, scaled ? P.mnfp : nullptr, nd, 1, nd, np, src, 1, np, ncol,
+             scaled ? ys : nullptr, np, (scaled && P.mnfp) ? gs.tg : nullptr, mat, nm, add, 1.0, out, sn, sc_};
+    const bool own = bytes >= (long long)sizeof(gs.tile);
+    prod64_team(t, a, own ? region : (void *)gs.tile, own ? bytes : (long long)sizeof(gs.tile));
 }
 
 // zout[p,col] = Σ_n Dn[p,n]·ψ[n,col]   (matvec: zout = zin − that); FP32 product in the mixed
 // form, written to the FP64 state.
 template <class Team>
-__device__ void d2m_tiles(Team &t, const DevProblem &P, GroupShared &gs, const double *zin, double *zout, int matvec,
-                          int mixed = 0) {
+__device__ void d2m_tiles(Team &t, const DevProblem &P, GroupShared &gs, void *region, long long bytes,
+                          const double *zin, double *zout, int matvec, int mixed = 0) {
     const int nd = P.nd, np = P.np, nm = P.nm5;
-    auto one = [] __device__(int, long long) { return 1.0; };
-    auto pre = [=] __device__(int i, long long col) { return matvec ? zin[col * np + i] : 0.0; };
-    auto st = [=] __device__(int i, long long col, double v, double z) { zout[col * np + i] = matvec ? z - v : v; };
+    const long long ncol = (long long)nm * P.ncell;
     if (mixed) {
-        ProductArgs<float> a{P.dn, nullptr, np, np, nd, P.psi32, nd, (long long)nm * P.ncell};
+        auto one = [] __device__(int, long long) { return 1.0; };
+        auto pre = [=] __device__(int i, long long col) { return matvec ? zin[col * np + i] : 0.0; };
+        auto st = [=] __device__(int i, long long col, double v, double z) { zout[col * np + i] = matvec ? z - v : v; };
+        ProductArgs<float> a{P.dn, nullptr, np, np, nd, P.psi32, P.psi_sn, P.psi_sc, ncol};
         team_product<float>(t, gs, a, one, pre, st);
-    } else {
-        ProductArgs<double> a{P.dn, nullptr, np, np, nd, P.psi, nd, (long long)nm * P.ncell};
-        team_product<double>(t, gs, a, one, pre, st);
+        return;
     }
+    Prod64 a{P.dn, nullptr, np, 1, np, nd, P.psi, P.psi_sn, P.psi_sc, ncol, nullptr, 0, nullptr, P.mat, nm,
+             matvec ? zin : nullptr, matvec ? -1.0 : 1.0, zout, 1, np};
+    const bool own = bytes >= (long long)sizeof(gs.tile);
+    prod64_team(t, a, own ? region : (void *)gs.tile, own ? bytes : (long long)sizeof(gs.tile));
 }
 
 // ------------------------------------------------------------------------------------------
@@ -828,11 +838,11 @@ __device__ void d2m_tiles(Team &t, const DevProblem &P, GroupShared &gs, const d
 // matvec != 0 writes zout = zin − A·zin instead (the Krylov operator of sn_one_speed.jl:147).
 // ------------------------------------------------------------------------------------------
 template <class Team>
-__device__ void pass1d(Team &t, const DevProblem &P, GroupShared &gs, const double *zin, double *zout, int homog,
-                       int matvec, int ig, const double *phiE_in, double *phiE_out, int mixed = 0) {
+__device__ void pass1d(Team &t, const DevProblem &P, GroupShared &gs, void *region, long long bytes,
+                       const double *zin, double *zout, int homog, int matvec, int ig, const double *phiE_in,
+                       double *phiE_out, int mixed = 0) {
     const int nd = P.nd;
-    // M2D over column tiles staged in shared memory
-    m2d_tiles(t, P, gs, zin, homog ? nullptr : P.qnout, 1, mixed);
+    m2d_tiles(t, P, gs, region, bytes, zin, homog ? nullptr : P.qnout, P.psi, 1, mixed);
     t.sync();
     // sweep; homogeneous passes see no surface source and a zero incoming energy flux
     // (sn_inner_pass.jl:37-38)
@@ -841,8 +851,7 @@ __device__ void pass1d(Team &t, const DevProblem &P, GroupShared &gs, const doub
     const double *pE = (P.csd && !homog) ? phiE_in : nullptr;
     sweep1d(t, P, gs, zin_b, np_source, pE, phiE_out, ig, mixed);
     t.sync();
-    // D2M over column tiles staged in shared memory; direction order kept per output
-    d2m_tiles(t, P, gs, zin, zout, matvec, mixed);
+    d2m_tiles(t, P, gs, region, bytes, zin, zout, matvec, mixed);
     // outgoing boundary moments: side 1 (X+) collects μ ≥ 0, side 0 (X-) μ < 0
     const int nf = P.nmf[0], nps = P.npsurf;
     const long long nb = P.nb[0];

@@ -47,8 +47,8 @@ __host__ __device__ __forceinline__ long long local1d_slice(const DevProblem &P,
 
 // bytes of the local region a problem needs on a cluster of `ncta` CTAs: face maps, exit
 // fluxes, the group's in-group Σs per material and moment, the CSD cell blocks per material,
-// the width and material of each owned cell, then ψ of the owned cells (which the
-// Gram-Schmidt loop reuses for the basis vector in use) and the slice of w
+// the width and material of each owned cell, then ψ of the owned cells (which a Gram-Schmidt loop
+// may reuse for a basis vector) and the slice of w
 __host__ __device__ __forceinline__ int local1d_kent(const DevProblem &P) {  // doubles per cell operator
     const int nm = P.nm5, nf = P.nmf[0];
     return nm * nm + nm * nf + nf * nf;
@@ -59,7 +59,11 @@ __host__ __device__ __forceinline__ long long local1d_bytes(const DevProblem &P,
     const long long psi = (nd + 1) * nm * lc, sl = local1d_slice(P, ncta);
     return 16 + nd * (RB_LMAP + RB_SCAN_NF) * 8 + (long long)P.nmat * P.np * 8 + (long long)P.nmat * nm * nm * 8 +
            (long long)RB_LKEYS * nd * local1d_kent(P) * 8 + lc * 8 + 2 * ((lc * 4 + 15) & ~15LL) +
-           (with_w ? ((psi > sl ? psi : sl) + sl) * 8 : psi * 8);
+           (with_w ? (psi > sl ? psi : sl) + sl : psi) * 8;
+}
+// the FP64 product operators as prod_tiles reads them, kept in the region where they fit
+__host__ __device__ __forceinline__ long long local1d_op_bytes(const DevProblem &P) {
+    return prod_bytes(prod_nt(P.nd), P.np, P.mnfp ? 2 : 1) + prod_bytes(prod_nt(P.np), P.nd, 1);
 }
 
 // whether a problem takes the local pass on a cluster of `ncta` CTAs with `local_bytes` of
@@ -83,15 +87,16 @@ struct Local1D {
     int *nkey;      // kinds among the owned cells; 0 when more than RB_LKEYS (per-cell solves)
     double *ktab;   // [RB_LKEYS][nd][kent] factored cell operators: S⁻¹, S⁻¹·h·Gsrc, the face map
     int kent;
-    void *psi;      // [ncl][ldp] ψ of the local columns (double or float); in the Gram-Schmidt
-                    // loop, the slice of the basis vector in use
-    double *ws;     // the slice of w in the Gram-Schmidt loop
+    void *psi;      // [ncl][ldp] ψ of the local columns (double or float)
+    double *ws;     // the slice of w in the Gram-Schmidt loop (null: does not fit)
+    double *vb;     // the slice of the next basis vector (null: not mixed, or does not fit)
+    double *opM, *opD;  // resident FP64 operators of M2D and D2M (null: do not fit)
     long long ldp;  // leading dimension of ψ (nd + 1: odd, so column accesses spread over banks)
     int cb, ce;     // owned cells [cb, ce)
     long long e0, eb;  // slice element j < l1 is state element e0 + j, the rest eb + (j − l1)
     int l1, ls;        // length of the cell part and of the whole slice
 
-    __device__ Local1D(const DevProblem &P, unsigned crank, unsigned ncta, void *base) {
+    __device__ Local1D(const DevProblem &P, unsigned crank, unsigned ncta, void *base, long long bytes) {
         const int lc = (P.nx + (int)ncta - 1) / (int)ncta;
         cb = min(P.nx, (int)crank * lc);
         ce = min(P.nx, cb + lc);
@@ -107,8 +112,18 @@ struct Local1D {
         key = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(mat) + ((lc * 4 + 15) & ~15));
         psi = reinterpret_cast<unsigned char *>(key) + ((lc * 4 + 15) & ~15);
         ldp = P.nd + 1;
-        const long long np_ = (long long)(P.nd + 1) * P.nm5 * lc, sl = local1d_slice(P, (int)ncta);
-        ws = reinterpret_cast<double *>(psi) + (np_ > sl ? np_ : sl);
+        const long long np0 = (long long)(P.nd + 1) * P.nm5 * lc, sl = local1d_slice(P, (int)ncta);
+        const long long np_ = np0 > sl ? np0 : sl;
+        const bool w = local1d_bytes(P, (int)ncta, true) <= bytes;
+        ws = w ? reinterpret_cast<double *>(psi) + np_ : nullptr;
+        // the mixed form's Gram-Schmidt loop keeps the next basis vector's slice beside the one in work
+        const long long b0 = (local1d_bytes(P, (int)ncta, w) + 15) & ~15LL;
+        const bool next = w && P.precision == 1 && b0 + sl * 8 <= bytes;
+        vb = next ? reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(base) + b0) : nullptr;
+        const long long used = next ? (b0 + sl * 8 + 15) & ~15LL : b0;
+        const bool op = P.nd <= 8 * RB_PROD_MAXNT && P.np <= 8 * RB_PROD_MAXNT && used + local1d_op_bytes(P) <= bytes;
+        opM = op ? reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(base) + used) : nullptr;
+        opD = op ? opM + prod_bytes(prod_nt(P.nd), P.np, P.mnfp ? 2 : 1) / 8 : nullptr;
         e0 = (long long)P.np * P.nm5 * cb;
         eb = P.nphi;
         l1 = (int)((long long)P.np * P.nm5 * (ce - cb));
@@ -116,28 +131,22 @@ struct Local1D {
     }
 };
 
-// Loop over the CTA's slice of a Krylov vector: element j of the slice is state element g,
-// RB_SVU elements per thread in flight (a 4-CTA team's whole slice of a C2-sized state).
-#define RB_SVU 40
-#define RB_SLICE_LOOP(L, LOAD, USE)                                                         \
-    {                                                                                      \
-        const int l1_ = (L).l1, ls_ = (L).ls;                                              \
-        const long long e0_ = (L).e0, eb_ = (L).eb;                                        \
-        for (int j0_ = threadIdx.x; j0_ < ls_; j0_ += RB_SVU * blockDim.x) {               \
-            _Pragma("unroll") for (int u_ = 0; u_ < RB_SVU; u_++) {                         \
-                const int j = j0_ + u_ * blockDim.x;                                       \
-                const long long g = j < l1_ ? e0_ + j : eb_ + (j - l1_);                   \
-                if (j < ls_) { LOAD }                                                      \
-                (void)g;                                                                   \
-            }                                                                              \
-            _Pragma("unroll") for (int u_ = 0; u_ < RB_SVU; u_++) {                         \
-                const int j = j0_ + u_ * blockDim.x;                                       \
-                const long long g = j < l1_ ? e0_ + j : eb_ + (j - l1_);                   \
-                if (j < ls_) { USE }                                                       \
-                (void)g;                                                                   \
-            }                                                                              \
-        }                                                                                  \
-    }
+// state element of element j of the CTA's slice of a Krylov vector
+__device__ __forceinline__ long long local1d_elem(const Local1D &L, int j) {
+    return j < L.l1 ? L.e0 + j : L.eb + (j - L.l1);
+}
+
+// the FP64 operators into the region, once per problem
+__device__ __forceinline__ void local1d_load_ops(const DevProblem &P, Local1D &L) {
+    if (!L.opM) return;
+    Prod64 a{};
+    a.A = P.mn; a.B = P.mnfp; a.lda = P.nd; a.ldi = 1; a.ni = P.nd; a.nk = P.np;
+    prod_load_op(a, L.opM, 0, prod_nt(P.nd));
+    a.A = P.dn; a.B = nullptr; a.lda = P.np; a.ni = P.np; a.nk = P.nd;
+    prod_load_op(a, L.opD, 0, prod_nt(P.np));
+}
+
+static_assert(sizeof(Local1D) <= sizeof(GroupShared::l1d), "Local1D lives in GroupShared");
 
 // per-group copy of the tables the local pass reads per cell (after the group's constants are set)
 __device__ __forceinline__ void local1d_group_setup(const DevProblem &P, Local1D &L) {
@@ -329,7 +338,7 @@ struct CellKey1D {
                 R a = w1E * FE[e];
 #pragma unroll
                 for (int j = 0; j < NM; j++) a += (R)P.Eout[e + NE * j] * y[j];
-                phiE_out[n + (long long)nd * (e + (long long)NE * c)] = (double)a;
+                if (phiE_out) phiE_out[n + (long long)nd * (e + (long long)NE * c)] = (double)a;
             }
         }
         PS *pc = psi + n + L.ldp * NM * lc;
@@ -559,7 +568,8 @@ __device__ bool sweep1d_local_fixed(ClusterTeam &t, const DevProblem &P, GroupSh
 }
 
 // the products of the local pass, compiled as functions of their own so that their registers
-// are allocated apart from the rest of the solve
+// are allocated apart from the rest of the solve: FP64 on the FP64 tensor pipe (prod_tiles, the
+// operators resident where they fit), FP32 (mixed form) through team_product
 template <typename T, typename PS>
 __device__ __noinline__ void m2d_local(const DevProblem &P, GroupShared &gs, Local1D &L, const double *zin,
                                        int homog) {
@@ -574,15 +584,31 @@ __device__ __noinline__ void m2d_local(const DevProblem &P, GroupShared &gs, Loc
         const int *mat = L.mat;
         const double *ys = L.kmat;
         const double *add = homog ? nullptr : P.qnout;
-        ProductArgs<double> a{P.mn, P.mnfp, nd, nd, np, zin + (long long)np * col0, np, ncl};
-        auto sc = [=, &gs] __device__(int k, long long lc) {
-            const int m = mat[lc / nm];
-            return k < np ? ys[(long long)m * np + k] : gs.tg[m];
-        };
-        auto pre = [=] __device__(int i, long long lc) { return add ? add[(col0 + lc) * nd + i] : 0.0; };
-        team_product<T>(ct, gs, a, sc, pre, [=] __device__(int i, long long lc, double v, double ad) {
-            psi[i + ldp * lc] = (PS)(ad + v);
-        });
+        if constexpr (sizeof(PS) == 8) {
+            // the added term sits nd apart, ψ ldp apart: it is copied into ψ first
+            if (add)
+                for (int c = threadIdx.x >> 5; c < (int)ncl; c += blockDim.x >> 5)
+                    for (int n = threadIdx.x & 31; n < nd; n += 32) psi[n + ldp * c] = add[(col0 + c) * nd + n];
+            if (add) __syncthreads();
+            Prod64 a{P.mn, P.mnfp, nd, 1, nd, np, zin + (long long)np * col0, 1, np, ncl, ys, np,
+                     P.mnfp ? gs.tg : nullptr, mat, nm, add ? psi : nullptr, 1.0, psi, 1, ldp};
+            if (L.opM) {
+                prod_run(a, L.opM, 0, prod_nt(nd), threadIdx.x >> 5, blockDim.x >> 5);
+                __syncthreads();
+            } else {
+                prod64_team(ct, a, gs.tile, sizeof(gs.tile));
+            }
+        } else {
+            ProductArgs<double> a{P.mn, P.mnfp, nd, nd, np, zin + (long long)np * col0, 1, np, ncl};
+            auto sc = [=, &gs] __device__(int k, long long lc) {
+                const int m = mat[lc / nm];
+                return k < np ? ys[(long long)m * np + k] : gs.tg[m];
+            };
+            auto pre = [=] __device__(int i, long long lc) { return add ? add[(col0 + lc) * nd + i] : 0.0; };
+            team_product<T>(ct, gs, a, sc, pre, [=] __device__(int i, long long lc, double v, double ad) {
+                psi[i + ldp * lc] = (PS)(ad + v);
+            });
+        }
     }
 }
 
@@ -595,14 +621,25 @@ __device__ __noinline__ void d2m_local(const DevProblem &P, GroupShared &gs, Loc
     PS *psi = reinterpret_cast<PS *>(L.psi);
     const long long ldp = L.ldp;
     CtaTeam ct;
-    // D2M: 𝚽[p, col] = Σ_n Dn[p,n]·ψ[n, col], direction order kept per output
+    // D2M: 𝚽[p, col] = Σ_n Dn[p,n]·ψ[n, col]
     if (ncl > 0) {
-        ProductArgs<PS> a{P.dn, nullptr, np, np, nd, psi, (int)ldp, ncl};
-        auto one = [] __device__(int, long long) { return 1.0; };
-        auto pre = [=] __device__(int i, long long lc) { return matvec ? zin[(col0 + lc) * np + i] : 0.0; };
-        team_product<T>(ct, gs, a, one, pre, [=] __device__(int i, long long lc, double v, double z) {
-            zout[(col0 + lc) * np + i] = matvec ? z - v : v;
-        });
+        if constexpr (sizeof(PS) == 8) {
+            Prod64 a{P.dn, nullptr, np, 1, np, nd, psi, 1, ldp, ncl, nullptr, 0, nullptr, nullptr, nm,
+                     matvec ? zin + col0 * np : nullptr, matvec ? -1.0 : 1.0, zout + col0 * np, 1, np};
+            if (L.opD) {
+                prod_run(a, L.opD, 0, prod_nt(np), threadIdx.x >> 5, blockDim.x >> 5);
+                __syncthreads();
+            } else {
+                prod64_team(ct, a, gs.tile, sizeof(gs.tile));
+            }
+        } else {
+            ProductArgs<PS> a{P.dn, nullptr, np, np, nd, psi, 1, ldp, ncl};
+            auto one = [] __device__(int, long long) { return 1.0; };
+            auto pre = [=] __device__(int i, long long lc) { return matvec ? zin[(col0 + lc) * np + i] : 0.0; };
+            team_product<T>(ct, gs, a, one, pre, [=] __device__(int i, long long lc, double v, double z) {
+                zout[(col0 + lc) * np + i] = matvec ? z - v : v;
+            });
+        }
     }
 }
 
@@ -620,10 +657,10 @@ __device__ void pass1d_local_t(ClusterTeam &t, const DevProblem &P, GroupShared 
     t.sync();
 }
 
-__device__ __forceinline__ void pass1d_local(ClusterTeam &t, const DevProblem &P, GroupShared &gs, void *base,
+__device__ __forceinline__ void pass1d_local(ClusterTeam &t, const DevProblem &P, GroupShared &gs,
                                              const double *zin, double *zout, int homog, int matvec, int ig,
                                              const double *phiE_in, double *phiE_out, int mixed) {
-    Local1D L(P, t.crank, t.ncta, base);
+    Local1D &L = *reinterpret_cast<Local1D *>(gs.l1d);
     if (mixed) pass1d_local_t<float, float>(t, P, gs, L, zin, zout, homog, matvec, ig, phiE_in, phiE_out);
     else pass1d_local_t<double, double>(t, P, gs, L, zin, zout, homog, matvec, ig, phiE_in, phiE_out);
 }

@@ -52,19 +52,22 @@ struct Solver {
     // next group (the outer defect-correction update).
     // One copy of the pass per kernel (it is called from every accelerator): its own register
     // allocation, and a compile time that does not grow with the number of call sites.
-    __device__ __noinline__ void pass(const double *zin, double *out, int homog, int mv, int final = 0) {
+    // emit: the outgoing energy-face flux is written (the reconstruction pass alone: the others' is
+    // never read).
+    __device__ __noinline__ void pass(const double *zin, double *out, int homog, int mv, int final = 0, int emit = 0) {
         const int mixed = (P.precision == 1 && !final) ? 1 : 0;
+        double *phiE_out = emit ? this->phiE_out : nullptr;
         npass++;
         if constexpr (std::is_same<Team, ClusterTeam>::value) {
             if (LO || local_ok) {
-                pass1d_local(t, P, gs, local, zin, out, homog, mv, ig, phiE_in, phiE_out, mixed);
+                pass1d_local(t, P, gs, zin, out, homog, mv, ig, phiE_in, phiE_out, mixed);
                 return;
             }
         }
         if constexpr (std::is_same<Team, GridTeam>::value) {  // the grid team runs 2D/3D problems only
             pass_md(t, P, gs, local, local_bytes, zin, out, homog, mv, ig, phiE_in, phiE_out, mixed);
         } else if constexpr (!LO) {
-            if (P.ndims == 1) pass1d(t, P, gs, zin, out, homog, mv, ig, phiE_in, phiE_out, mixed);
+            if (P.ndims == 1) pass1d(t, P, gs, local, local_bytes, zin, out, homog, mv, ig, phiE_in, phiE_out, mixed);
             else pass_md(t, P, gs, local, local_bytes, zin, out, homog, mv, ig, phiE_in, phiE_out, mixed);
         }
     }
@@ -206,59 +209,334 @@ struct Solver {
         return s;
     }
 
-    // Modified Gram-Schmidt of w against V_0..V_j for a problem on the local 1D pass: each CTA
-    // keeps its slice of w, and of the basis vector in use, in shared memory, so a step reads
-    // only the next basis vector from memory. Same steps and fused dot products as the
-    // team-wide loop in gmres; writes H[0..j, j] and V_{j+1}, returns false when not local.
-    __device__ __noinline__ bool mgs_local(const double *w, int jb, int m, double &hjp1) {
-        if constexpr (std::is_same<Team, ClusterTeam>::value) {
-            if (!local_w) return false;
-            Local1D L(P, t.crank, t.ncta, local);
-            double *ws = L.ws, *vs = reinterpret_cast<double *>(L.psi);
-            double *H = gs.H;
-            {
-                const double *V0 = vec(4);
-                double acc[1] = {0.0};
-                double xw[RB_SVU], xv[RB_SVU];
-                RB_SLICE_LOOP(L, { xw[u_] = w[g]; xv[u_] = V0[g]; }, {
-                    ws[j] = xw[u_];
-                    vs[j] = xv[u_];
-                    acc[0] += xw[u_] * xv[u_];
-                })
-                t.template sumk<1>(acc);
-                double h = acc[0];
-                for (int i = 0; i <= jb; i++) {
-                    if (t.leader()) H[i + (m + 1) * jb] = h;
-                    double a1[1] = {0.0};
-                    if (i < jb) {
-                        const double *Vn = vec(4 + i + 1);
-                        double xn[RB_SVU];
-                        RB_SLICE_LOOP(L, { xn[u_] = Vn[g]; }, {
-                            const double wq = ws[j] + (-h) * vs[j];
-                            ws[j] = wq;
-                            vs[j] = xn[u_];
-                            a1[0] += wq * xn[u_];
-                        })
-                    } else {
-                        RB_SLICE_LOOP(L, {}, {
-                            const double wq = ws[j] + (-h) * vs[j];
-                            ws[j] = wq;
-                            a1[0] += wq * wq;
-                        })
-                    }
-                    t.template sumk<1>(a1);
-                    h = a1[0];
+    // Modified Gram-Schmidt of w against V_0..V_jb (gmres.jl) in two reductions instead of jb + 2.
+    // The coefficients of the modified form, h_i = V_i·(w − Σ_{k<i} h_k V_k), are the solution of
+    // (I + L)·h = Vᵀw with L the strictly lower part of VᵀV (Świrydowicz, Langou, Ananthan, Yang and
+    // Thomas 2021, "Low synchronization Gram-Schmidt and GMRES algorithms"): same projection and same
+    // stability, every inner product from one pass over the basis, and no basis vector's load waits
+    // for a reduction. L's row of V_jb comes with the products of w and stays below the diagonal of
+    // H, which the Givens rotations leave free. Writes H[0..jb, jb] and V_{jb+1}; returns
+    // H[jb+1, jb].
+    //
+    // Each thread takes elements q0, q0 + blockDim.x, … < q1 (of type E: a double or an aligned
+    // pair); Krylov vectors hold element q at [q], w is read at w0 and written at w1 (shared memory
+    // on the local 1D pass).
+    static __device__ __forceinline__ double dot_add(double s, double a, double b) { return s + a * b; }
+    static __device__ __forceinline__ double dot_add(double s, double2 a, double2 b) { return (s + a.x * b.x) + a.y * b.y; }
+    static __device__ __forceinline__ double minus(double a, double h, double v) { return a - h * v; }
+    static __device__ __forceinline__ double2 minus(double2 a, double h, double2 v) {
+        return make_double2(a.x - h * v.x, a.y - h * v.y);
+    }
+    static __device__ __forceinline__ double times(double a, double s) { return a * s; }
+    static __device__ __forceinline__ double2 times(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
+
+    // acc[e] += V_{i0+e}·w and acc[4+e] += V_{i0+e}·V_jb over this thread's elements: four basis
+    // vectors at a time, U elements' loads in flight together
+    template <typename E, int U>
+    static __device__ __forceinline__ void mgs_dots(const E *w, const E *vj, const E *const (&V)[4], int q0, int q1,
+                                                    double (&acc)[8]) {
+        const int step = blockDim.x;
+        int q = q0;
+        for (; q + (U - 1) * step < q1; q += U * step) {
+            E xw[U], xj[U], xv[U][4];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                xw[u] = w[q + u * step];
+                xj[u] = vj[q + u * step];
+#pragma unroll
+                for (int e = 0; e < 4; e++) xv[u][e] = V[e][q + u * step];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    acc[e] = dot_add(acc[e], xw[u], xv[u][e]);
+                    acc[4 + e] = dot_add(acc[4 + e], xj[u], xv[u][e]);
                 }
-                hjp1 = sqrt(h);
-                if (hjp1 > 0.0) {
-                    const double inv = 1.0 / hjp1;
-                    double *Vn = vec(4 + jb + 1);
-                    RB_SLICE_LOOP(L, {}, { Vn[g] = ws[j] * inv; })
+        }
+        for (; q < q1; q += step) {
+            E x[6] = {w[q], vj[q], V[0][q], V[1][q], V[2][q], V[3][q]};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                acc[e] = dot_add(acc[e], x[0], x[2 + e]);
+                acc[4 + e] = dot_add(acc[4 + e], x[1], x[2 + e]);
+            }
+        }
+    }
+
+    // w1 = w0 − Σ h_i V_i over this thread's elements; returns its part of ‖w1‖²
+    template <typename E, int U>
+    static __device__ __forceinline__ double mgs_update(const E *w0, E *w1, const E *V0, long long ldv, int q0, int q1, int n,
+                                                        const double *h) {
+        const int step = blockDim.x;
+        double s = 0.0;
+        for (int q = q0; q < q1; q += U * step) {
+            E x[U];
+            int g[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                g[u] = q + u * step < q1 ? q + u * step : q;
+                x[u] = w0[g[u]];
+            }
+            int i = 0;
+            for (; i + 4 <= n; i += 4) {
+                E v[4][U];
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+#pragma unroll
+                    for (int u = 0; u < U; u++) v[e][u] = V0[(i + e) * ldv + g[u]];
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+#pragma unroll
+                    for (int u = 0; u < U; u++) x[u] = minus(x[u], h[i + e], v[e][u]);
+            }
+            if (i < n) {
+                E v[3][U];
+#pragma unroll
+                for (int e = 0; e < 3; e++)
+#pragma unroll
+                    for (int u = 0; u < U; u++) v[e][u] = V0[min(i + e, n - 1) * ldv + g[u]];
+#pragma unroll
+                for (int e = 0; e < 3; e++)
+                    if (i + e < n)
+#pragma unroll
+                        for (int u = 0; u < U; u++) x[u] = minus(x[u], h[i + e], v[e][u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (q + u * step < q1) {
+                    w1[g[u]] = x[u];
+                    s = dot_add(s, x[u], x[u]);
+                }
+        }
+        return s;
+    }
+
+    template <typename E>
+    static __device__ __forceinline__ void mgs_scale(const E *w, E *v, double inv, int q0, int q1) {
+        const int step = blockDim.x;
+        for (int q = q0; q < q1; q += 4 * step) {
+            E x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (q + u * step < q1) x[u] = w[q + u * step];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (q + u * step < q1) v[q + u * step] = times(x[u], inv);
+        }
+    }
+
+    // h from b = Vᵀw by forward substitution with I + L (one warp, a row or two per lane)
+    __device__ __forceinline__ void mgs_coefficients(double *b, int n, int m) {
+        double *H = gs.H;
+        const int jb = n - 1, lane = threadIdx.x & 31;
+        if (threadIdx.x < 32) {
+            for (int i = lane; i < jb; i += 32) H[jb + (m + 1) * i] = b[n + i];
+            __syncwarp();
+            double b0 = lane < n ? b[lane] : 0.0, b1 = lane + 32 < n ? b[lane + 32] : 0.0;
+            for (int k = 0; k < jb; k++) {
+                const double hk = __shfl_sync(0xffffffffu, k < 32 ? b0 : b1, k & 31);
+                if (lane > k && lane < n) b0 -= H[lane + (m + 1) * k] * hk;
+                if (lane + 32 > k && lane + 32 < n) b1 -= H[lane + 32 + (m + 1) * k] * hk;
+            }
+            if (lane < n) { b[lane] = b0; H[lane + (m + 1) * jb] = b0; }
+            if (lane + 32 < n) { b[lane + 32] = b1; H[lane + 32 + (m + 1) * jb] = b1; }
+        }
+        __syncthreads();
+    }
+
+    // The mixed form keeps the modified form step by step (its FP32 roundings follow the last bit of
+    // every coefficient): w − h_i V_i fused with the product of the next basis vector. On the local 1D
+    // pass w, V_i and V_{i+1} are slices in shared memory (ψ's region is free meanwhile), V_{i+1}
+    // copied asynchronously while the reduction of h_i is under way: short rolled loops, no register
+    // arrays (40 elements a thread in registers spilled, and the unrolled loops took 40 predicated
+    // turns for slices of 3). Where the third slice does not fit, V_{i+1} is loaded in the update.
+    __device__ __noinline__ double mgs_ordered(double *w, int jb, int m) {
+        const Local1D &L = *reinterpret_cast<const Local1D *>(gs.l1d);
+        const long long ldv = P.vstride, e0 = L.e0, eb = L.eb - L.l1;
+        const double *V = vec(4);
+        const int ls = L.ls, l1 = L.l1, tid = threadIdx.x;
+        constexpr int step = RB_THREADS;
+        double *ws = L.ws, *va = reinterpret_cast<double *>(L.psi), *vb = L.vb, acc[1] = {0.0};
+        auto at = [=](int j) -> long long { return (j < l1 ? e0 : eb) + j; };
+        auto copy = [&](double *dst, const double *src) {
+#pragma unroll 4
+            for (int j = tid; j < ls; j += step) cp_zfill<8>(dst + j, src + at(j), true);
+        };
+        auto landed = [] {
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        };
+        copy(ws, w);
+        copy(va, V);
+        landed();
+#pragma unroll 8
+        for (int j = tid; j < ls; j += step) acc[0] += ws[j] * va[j];
+        for (int i = 0; i <= jb; i++) {
+            const double *Vn = V + (i + 1) * ldv;
+            if (vb && i < jb) copy(vb, Vn);
+            t.template sumk<1>(acc);
+            const double h = acc[0];
+            if (t.leader()) gs.H[i + (m + 1) * jb] = h;
+            acc[0] = 0.0;
+            landed();
+            if (i == jb) {
+#pragma unroll 8
+                for (int j = tid; j < ls; j += step) {
+                    const double x = ws[j] + (-h) * va[j];
+                    ws[j] = x;
+                    acc[0] += x * x;
+                }
+            } else if (vb) {
+#pragma unroll 8
+                for (int j = tid; j < ls; j += step) {
+                    const double x = ws[j] + (-h) * va[j];
+                    ws[j] = x;
+                    acc[0] += x * vb[j];
+                }
+                double *s = va;
+                va = vb;
+                vb = s;
+            } else {
+                for (int j0 = tid; j0 < ls; j0 += 8 * step) {
+                    double b[8];
+#pragma unroll
+                    for (int u = 0; u < 8; u++)
+                        if (j0 + u * step < ls) b[u] = Vn[at(j0 + u * step)];
+#pragma unroll
+                    for (int u = 0; u < 8; u++)
+                        if (j0 + u * step < ls) {
+                            const int j = j0 + u * step;
+                            const double x = ws[j] + (-h) * va[j];
+                            ws[j] = x;
+                            va[j] = b[u];
+                            acc[0] += x * b[u];
+                        }
                 }
             }
-            return true;
         }
-        return false;
+        t.template sumk<1>(acc);
+        const double hn = sqrt(acc[0]);
+        if (hn > 0.0) {
+            const double inv = 1.0 / hn;
+            double *Vo = vec(4 + jb + 1);
+#pragma unroll 4
+            for (int j = tid; j < ls; j += step) Vo[at(j)] = ws[j] * inv;
+        }
+        return hn;
+    }
+    // the same over 16-byte pairs of the CTA's contiguous range
+    __device__ __forceinline__ double mgs_ordered_pairs(double *w, int jb, int m) {
+        const long long N2 = P.vstride / 2;
+        double h = vdot2(t, w, vec(4), N2);
+        double2 *w2 = RB_D2(w);
+        for (int i = 0; i <= jb; i++) {
+            if (t.leader()) gs.H[i + (m + 1) * jb] = h;
+            const double2 *Vi2 = RB_CD2(vec(4 + i)), *Vn2 = i < jb ? RB_CD2(vec(4 + i + 1)) : nullptr;
+            double acc[1] = {0.0};
+            double2 xw[4], xv[4], xn[4];
+            if (Vn2) {
+                RB_VPAIRS_D(t, N2, 4, { xw[u_] = w2[q]; xv[u_] = Vi2[q]; xn[u_] = Vn2[q]; }, {
+                    double2 wq;
+                    wq.x = xw[u_].x + (-h) * xv[u_].x;
+                    wq.y = xw[u_].y + (-h) * xv[u_].y;
+                    w2[q] = wq;
+                    acc[0] += wq.x * xn[u_].x;
+                    acc[0] += wq.y * xn[u_].y;
+                })
+            } else {
+                RB_VPAIRS_D(t, N2, 4, { xw[u_] = w2[q]; xv[u_] = Vi2[q]; }, {
+                    double2 wq;
+                    wq.x = xw[u_].x + (-h) * xv[u_].x;
+                    wq.y = xw[u_].y + (-h) * xv[u_].y;
+                    w2[q] = wq;
+                    acc[0] += wq.x * wq.x;
+                    acc[0] += wq.y * wq.y;
+                })
+            }
+            t.template sumk<1>(acc);
+            h = acc[0];
+        }
+        const double hn = sqrt(h);
+        if (hn > 0.0) {
+            const double inv = 1.0 / hn;
+            double2 *Vn2 = RB_D2(vec(4 + jb + 1));
+            double2 xw[4];
+            RB_VPAIRS_D(t, N2, 4, { xw[u_] = w2[q]; }, { Vn2[q] = make_double2(xw[u_].x * inv, xw[u_].y * inv); })
+        }
+        return hn;
+    }
+    __device__ __noinline__ double gram_schmidt_ordered(double *w, int jb, int m) {
+        if constexpr (std::is_same<Team, ClusterTeam>::value) {
+            if (local_w) return mgs_ordered(w, jb, m);
+        }
+        return mgs_ordered_pairs(w, jb, m);
+    }
+
+    // The CTA's share of a Krylov vector as up to two runs of doubles: [g0, g0 + n0) and, in the last
+    // CTA of a local 1D problem, the boundary moments [g1, g1 + n1).
+    __device__ __noinline__ double gram_schmidt(double *w, int jb, int m) {
+        const int n = jb + 1, warp = threadIdx.x >> 5, tid = threadIdx.x;
+        const long long ldv = P.vstride;
+        double *V = vec(4), *ws = nullptr;
+        long long g0, g1 = 0;
+        int n0, n1 = 0;
+        if (std::is_same<Team, ClusterTeam>::value && local_w) {
+            const Local1D &L = *reinterpret_cast<const Local1D *>(gs.l1d);
+            ws = L.ws;
+            g0 = L.e0; n0 = L.l1; g1 = L.eb; n1 = L.ls - L.l1;
+        } else {
+            const long long np_ = ldv / 2;
+            g0 = 2 * (np_ * t.crank / t.ncta);
+            n0 = (int)(2 * (np_ * (t.crank + 1) / t.ncta) - g0);
+        }
+        double *u = ws ? ws - g0 : w;  // w after the first update, by position (run 1: shifted)
+        double *u1 = ws ? ws + n0 - g1 : w;
+        const bool pair = g0 % 2 == 0 && n0 % 2 == 0 && reinterpret_cast<uintptr_t>(u + g0) % 16 == 0;
+        for (int i0 = 0; i0 < n; i0 += 4) {
+            double acc[8] = {};
+            const double *Ve[4];
+            const double2 *Ve2[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                Ve[e] = V + min(i0 + e, jb) * ldv + g0;
+                Ve2[e] = RB_CD2(Ve[e]);
+            }
+            const double *vj = V + jb * ldv;
+            if (pair) mgs_dots<double2, 2>(RB_CD2(w + g0), RB_CD2(vj + g0), Ve2, tid, n0 / 2, acc);
+            else mgs_dots<double, 4>(w + g0, vj + g0, Ve, tid, n0, acc);
+            if (n1 > 0) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) Ve[e] += g1 - g0;
+                mgs_dots<double, 1>(w + g1, vj + g1, Ve, tid, n1, acc);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int e = 0; e < 8; e++) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+            if ((tid & 31) == 0)
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    if (i0 + e < n) gs.red[warp * RB_SM + i0 + e] = acc[e];
+                    if (i0 + e < jb) gs.red[warp * RB_SM + n + i0 + e] = acc[4 + e];
+                }
+        }
+        double *h = t.sum_many(gs.red, 2 * n - 1);
+        mgs_coefficients(h, n, m);
+        double v[1];
+        if (pair) v[0] = mgs_update<double2, 2>(RB_CD2(w + g0), RB_D2(u + g0), RB_CD2(V + g0), ldv / 2, tid, n0 / 2, n, h);
+        else v[0] = mgs_update<double, 4>(w + g0, u + g0, V + g0, ldv, tid, n0, n, h);
+        if (n1 > 0) v[0] += mgs_update<double, 1>(w + g1, u1 + g1, V + g1, ldv, tid, n1, n, h);
+        t.template sumk<1>(v);
+        const double hn = sqrt(v[0]);
+        if (hn > 0.0) {
+            const double inv = 1.0 / hn;
+            double *Vn = V + n * ldv;
+            if (pair) mgs_scale<double2>(RB_CD2(u + g0), RB_D2(Vn + g0), inv, tid, n0 / 2);
+            else mgs_scale<double>(u + g0, Vn + g0, inv, tid, n0);
+            if (n1 > 0) mgs_scale<double>(u1 + g1, Vn + g1, inv, tid, n1);
+        }
+        return hn;
     }
 
     // ---------------------------------------------------------------- gmres(m)
@@ -310,48 +588,7 @@ struct Solver {
             for (int j = 0; j < m; j++) {
                 if (iter >= maxit) break;
                 matvec(w, vec(4 + j)); iter++;
-                double hjp1;
-                if (!mgs_local(w, j, m, hjp1)) {
-                // modified Gram-Schmidt, one sweep per basis vector: w ← w − h_i V_i fused with
-                // the dot product of the updated w against V_{i+1} (or against itself at the end)
-                double h = vdot2(t, w, vec(4), N2);
-                double2 *w2 = RB_D2(w);
-                for (int i = 0; i <= j; i++) {
-                    if (t.leader()) HH(i, j) = h;
-                    const double2 *Vi2 = RB_CD2(vec(4 + i));
-                    const double2 *Vn2 = (i < j) ? RB_CD2(vec(4 + i + 1)) : nullptr;
-                    double acc[1] = {0.0};
-                    double2 xw[RB_VU2], xv[RB_VU2], xn[RB_VU2];
-                    if (Vn2) {
-                        RB_VPAIRS(t, N2, { xw[u_] = w2[q]; xv[u_] = Vi2[q]; xn[u_] = Vn2[q]; }, {
-                            double2 wq;
-                            wq.x = xw[u_].x + (-h) * xv[u_].x;
-                            wq.y = xw[u_].y + (-h) * xv[u_].y;
-                            w2[q] = wq;
-                            acc[0] += wq.x * xn[u_].x;
-                            acc[0] += wq.y * xn[u_].y;
-                        })
-                    } else {
-                        RB_VPAIRS(t, N2, { xw[u_] = w2[q]; xv[u_] = Vi2[q]; }, {
-                            double2 wq;
-                            wq.x = xw[u_].x + (-h) * xv[u_].x;
-                            wq.y = xw[u_].y + (-h) * xv[u_].y;
-                            w2[q] = wq;
-                            acc[0] += wq.x * wq.x;
-                            acc[0] += wq.y * wq.y;
-                        })
-                    }
-                    t.template sumk<1>(acc);
-                    h = acc[0];
-                }
-                hjp1 = sqrt(h);
-                if (hjp1 > 0.0) {
-                    const double inv = 1.0 / hjp1;
-                    double2 *Vn2 = RB_D2(vec(4 + j + 1));
-                    double2 xw[RB_VU2];
-                    RB_VPAIRS(t, N2, { xw[u_] = w2[q]; }, { Vn2[q] = make_double2(xw[u_].x * inv, xw[u_].y * inv); })
-                }
-                }
+                const double hjp1 = P.precision == 1 ? gram_schmidt_ordered(w, j, m) : gram_schmidt(w, j, m);
                 if (t.leader()) {
                     HH(j + 1, j) = hjp1;
                     for (int i = 0; i < j; i++) {
@@ -580,7 +817,7 @@ struct Solver {
         }
         // reconstruction pass (sn_one_speed.jl:184-187)
         double *out = vec(1);
-        pass(z, out, 0, 0, 1);
+        pass(z, out, 0, 0, 1, 1);
         vcopy(t, flux_g, out, nphi);
         return st;
     }
@@ -590,8 +827,11 @@ struct Solver {
 // the group loop of compute_flux(::SN) for one problem (sn_flux.jl:146-224)
 // ------------------------------------------------------------------------------------------
 template <class Team, bool LO = false>
-__device__ void solve_problem(Team &t, const DevProblem &P, GroupShared &gs, void *local = nullptr,
+__device__ void solve_problem(Team &t, const DevProblem &P0, GroupShared &gs, void *local = nullptr,
                               long long local_bytes = 0) {
+    if (threadIdx.x == 0) gs.prob = P0;
+    __syncthreads();
+    const DevProblem &P = gs.prob;
     const int local_ok = (local && local1d_ok(P, (int)t.ncta, local_bytes)) ? 1 : 0;
     const int local_w = (local && local1d_w(P, (int)t.ncta, local_bytes)) ? 1 : 0;
     const int ng = P.ng, nmat = P.nmat, np = P.np, nd = P.nd, nm = P.nm5;
@@ -607,6 +847,14 @@ __device__ void solve_problem(Team &t, const DevProblem &P, GroupShared &gs, voi
     if (P.ndims == 3)
         for (int k = t.rank(); k < RB_OCT_MAXCTA; k += t.size()) P.oct_flags[k] = 0ull;
     if (threadIdx.x == 0) gs.oct_epoch = 0;
+    if constexpr (std::is_same<Team, ClusterTeam>::value) {
+        if (LO || local_ok) {
+            Local1D &L = *reinterpret_cast<Local1D *>(gs.l1d);
+            if (threadIdx.x == 0) L = Local1D(P, t.crank, t.ncta, local, local_bytes);
+            __syncthreads();
+            local1d_load_ops(P, L);
+        }
+    }
     t.sync();
     long long npass = 0;
     for (int ig = 0; ig < ng; ig++) {
@@ -668,15 +916,19 @@ __device__ void solve_problem(Team &t, const DevProblem &P, GroupShared &gs, voi
         t.sync();
         if constexpr (std::is_same<Team, ClusterTeam>::value) {
             if (LO || local_ok) {
-                Local1D L(P, t.crank, t.ncta, local);
+                Local1D &L = *reinterpret_cast<Local1D *>(gs.l1d);
                 local1d_group_setup(P, L);
                 local1d_factor_fixed(P, gs, L);
             }
         }
-        // Mn·Qlout into ψ, then kept as Qnout for the passes of this group
-        m2d_tiles(t, P, gs, P.qlout, nullptr, 0);
+        // Qnout = Mn·Qlout, kept for the passes of this group. The local 1D pass holds its region:
+        // the product stages in GroupShared there.
+        {
+            const bool own = local != nullptr && !(LO || local_ok);
+            m2d_tiles(t, P, gs, own ? local : (void *)gs.tile, own ? local_bytes : (long long)sizeof(gs.tile), P.qlout,
+                      nullptr, P.qnout, 0);
+        }
         t.sync();
-        vcopy(t, P.qnout, P.psi, (long long)nd * nm * ncell);
         Solver<Team, LO> S{t, P, gs, ig, phiE_in, phiE_out, 0};
         S.local = local;
         S.local_bytes = local ? local_bytes : 0;
@@ -700,7 +952,7 @@ __device__ void solve_problem(Team &t, const DevProblem &P, GroupShared &gs, voi
             double s = 0.0;
             if (is < P.nm4)
                 for (int n = 0; n < nd; n++)
-                    s += P.dn[p + (long long)np * n] * phiE_in[n + (long long)nd * (is + (long long)P.nm4 * c)];
+                    s += P.dn[p + (long long)np * n] * phiE_in[n * P.pe_sn + (is + (long long)P.nm4 * c) * P.psi_sc];
             P.cutoff[o] = s;
         }
     }

@@ -200,28 +200,92 @@ __device__ __forceinline__ long long md_in_offset(const DevProblem &P, int a) {
     return (a == 0 ? base : (a == 1 ? base + ny * nz : base + ny * nz + nx * nz)) * P.nfmax;
 }
 
-// The incoming face flux of every direction on every boundary face cell it enters through
-// (boundary_in_md: surface source plus the lagged reflective / periodic in-moments), as one
-// team phase before the sweep, so that the sweep reads one value per face cell instead of a
-// half-range sum per cell and direction.
-template <class Team>
-__device__ void boundary_in_phase(Team &t, const DevProblem &P, const double *zin, int np_source, int ig) {
-    const long long sstride = md_scratch_stride(P);
-    const int nfm = P.nfmax;
-    for (int a = 0; a < P.ndims; a++) {
-        const long long nfc = P.fcells[a];
-        const int nf = P.nmf[a];
-        const long long off = md_in_offset(P, a);
-        for (long long o = t.rank(); o < (long long)P.nd * nfc; o += t.size()) {
-            const int n = (int)(o / nfc);
-            const long long fc = o % nfc;
-            const bool fwd = P.cosv[(long long)a * P.nd + n] >= 0.0;
-            double f0[RB_MAXFACE];
-            boundary_in_md(P, n, a, fwd, fc, zin, np_source, ig, f0, nf);
-            double *dst = P.fexit + (long long)n * sstride + off + fc * nfm;
-            for (int f = 0; f < nf; f++) dst[f] = f0[f];
-        }
+// Part of a team, for products that run side by side.
+struct SubTeam {
+    unsigned crank, ncta;
+};
+// The item (axis, side, face moment) of index c of the faces' products, and how many there are.
+__device__ __forceinline__ int face_items(const DevProblem &P) {
+    int n = 0;
+    for (int a = 0; a < P.ndims; a++) n += 2 * P.nmf[a];
+    return n;
+}
+__device__ __forceinline__ void face_item(const DevProblem &P, int c, int &axis, int &side, int &is) {
+    axis = 0;
+    while (c >= 2 * P.nmf[axis]) c -= 2 * P.nmf[axis++];
+    side = c & 1;
+    is = c >> 1;
+}
+// Calls f(sub-team, axis, side, face moment) for every item, the items side by side on the team's
+// CTAs where there are enough of them.
+template <class Team, class F>
+__device__ __forceinline__ void for_faces(const Team &t, const DevProblem &P, F f) {
+    const int items = face_items(P), par = min(items, (int)t.ncta);
+    for (int c = (int)t.crank % par; c < items; c += par) {
+        int axis, side, is;
+        face_item(P, c, axis, side, is);
+        const int mine = (int)t.crank % par;
+        f(SubTeam{t.crank / par, (t.ncta - mine + par - 1) / par}, axis, side, is);
     }
+}
+
+// The incoming face flux of every direction on every boundary face cell it enters through
+// (boundary_in_md: surface source plus the lagged reflective / periodic in-moments), as one team
+// phase before the sweep, so that the sweep reads one value per face cell instead of a half-range
+// sum per cell and direction. Face by face and moment by moment it is a product of the half-range
+// rows with the face's moments (or source moments), and runs as one (64³, S8, reflective Z-: 62 us
+// as a sum per direction and cell, whose lanes each walked a cell's moments).
+template <class Team>
+__device__ __noinline__ void boundary_in_phase(Team &t, const DevProblem &P, void *region, long long bytes, const double *zin,
+                                               int np_source, int ig) {
+    const long long sstride = md_scratch_stride(P);
+    const int nfm = P.nfmax, nps = P.npsurf, nd = P.nd;
+    for_faces(t, P, [&](SubTeam st, int a, int side, int is) {
+        const int nf = P.nmf[a], face = 2 * a + side;
+        const long long nfc = P.fcells[a];
+        double *dst = P.fexit + md_in_offset(P, a) + is;
+        const double *cosv = P.cosv + (long long)a * nd;
+        const double *src = (is == 0 && np_source > 0) ? P.surf[face] : nullptr;
+        const int bcv = P.bc[face];
+        if ((src != nullptr) == (bcv != 0)) {  // neither, or (rare) both: per direction and cell
+            const long long np_ = st.ncta * (long long)blockDim.x;
+            for (long long o = st.crank * (long long)blockDim.x + threadIdx.x; o < nd * nfc; o += np_) {
+                const int n = (int)(o / nfc);
+                const long long fc = o - n * nfc;
+                if ((cosv[n] >= 0.0) != (side == 0)) continue;
+                double f0[RB_MAXFACE];
+                f0[is] = 0.0;
+                if (src) boundary_in_md(P, n, a, side == 0, fc, zin, np_source, ig, f0, nf);
+                dst[(long long)n * sstride + fc * nfm] = f0[is];
+            }
+            return;
+        }
+        Prod64 p{};
+        p.A = P.frow_m + (long long)a * nd * nps;  // [n][p]: rows n, k = p
+        p.lda = 1;
+        p.ldi = nps;
+        p.ni = nd;
+        if (src) {
+            p.nk = np_source;
+            p.X = src + ig;
+            p.sx = P.ng;
+            p.ldx = (long long)P.ng * np_source;
+        } else {
+            p.nk = nps;
+            p.X = zin + P.off_b[a] + (long long)nps * (is + (long long)nf * (bcv == 1 ? side : 1 - side));
+            p.sx = 1;
+            p.ldx = 2LL * nps * nf;
+        }
+        p.ncol = nfc;
+        p.nm = 1;
+        p.alpha = 1.0;
+        p.out = dst;
+        p.so = sstride;
+        p.ldo = nfm;
+        p.sel = cosv;
+        p.selpos = side == 0;
+        prod64_team(st, p, region, bytes);
+    });
 }
 
 // 3D: pencils along x in tiles of TY×TZ (one thread per pencil). Inside a tile the cells form a
@@ -317,7 +381,7 @@ __device__ void sweep_3d_tiles(Team &t, const DevProblem &P, GroupShared &gs, co
                                 FE[e] = phiE_in ? phiE_in[n + (long long)nd * (e + (long long)ne * c)] : 0.0;
                         Cell::step(P, gs, n, h, m, Qn, F, FE);
                         for (int j = 0; j < nm; j++) pc[(long long)nd * j] = Qn[j];
-                        if (P.csd)
+                        if (P.csd && phiE_out)
                             for (int e = 0; e < ne; e++) phiE_out[n + (long long)nd * (e + (long long)ne * c)] = FE[e];
                         if (smf) {
                             sfy[wr + me] = F[1][0];
@@ -398,15 +462,15 @@ __device__ void sweep_md(Team &t, const DevProblem &P, GroupShared &gs, const do
                         h[0] = fabs(mu) / P.dx[ix];
                         h[1] = fabs(eta) / P.dy[iy];
                         h[2] = nax == 3 ? fabs(xi) / P.dz[iz] : 0.0;
-                        double *pc = P.psi + n + (long long)nd * nm * c;
-                        for (int j = 0; j < nm; j++) Qn[j] = pc[(long long)nd * j];
+                        double *pc = P.psi + n * P.psi_sn + nm * c * P.psi_sc;
+                        for (int j = 0; j < nm; j++) Qn[j] = pc[j * P.psi_sc];
                         if (P.csd)
                             for (int e = 0; e < ne; e++)
-                                FE[e] = phiE_in ? phiE_in[n + (long long)nd * (e + (long long)ne * c)] : 0.0;
+                                FE[e] = phiE_in ? phiE_in[n * P.pe_sn + (e + (long long)ne * c) * P.psi_sc] : 0.0;
                         Cell::step(P, gs, n, h, m, Qn, F, FE);
-                        for (int j = 0; j < nm; j++) pc[(long long)nd * j] = Qn[j];
-                        if (P.csd)
-                            for (int e = 0; e < ne; e++) phiE_out[n + (long long)nd * (e + (long long)ne * c)] = FE[e];
+                        for (int j = 0; j < nm; j++) pc[j * P.psi_sc] = Qn[j];
+                        if (P.csd && phiE_out)
+                            for (int e = 0; e < ne; e++) phiE_out[n * P.pe_sn + (e + (long long)ne * c) * P.psi_sc] = FE[e];
                         for (int f = 0; f < nfy; f++) yf[(long long)ixx * nfy + f] = F[1][f];
                         if (nax == 3) {
                             if (izz < nz - 1)
@@ -427,107 +491,41 @@ __device__ void sweep_md(Team &t, const DevProblem &P, GroupShared &gs, const do
 }
 
 // Outgoing boundary moments of every face: b[p,is,side,cell] = Σ_n Dn_face[n][p]·exit[n][cell][is]
-// over the directions leaving through that side (sn_sweep_2D.jl:146-179, accumulated over n in
-// order as sn_inner_pass.jl:127-129 does).
-//
-// One thread per (face cell, face moment, side, block of PB half-range moments), neighbouring
-// lanes on neighbouring face cells: the exit loads of a warp are contiguous and its cosine and
-// half-range row loads are one address (one request, no divergence). The loads of 8 directions
-// go out together; a direction leaving through the other side enters with weight 0, which adds
-// exactly zero, so each moment is the sum over its side's directions in increasing n, as with one
-// thread per output. PB trades exit re-reads against threads (boundary_out_md picks it).
-template <int PB, class Team>
-__device__ void boundary_out_pb(Team &t, const DevProblem &P, const double *zin, double *zout, int matvec) {
-    const int nd = P.nd, nps = P.npsurf, nfm = P.nfmax;
-    const int npb = (nps + PB - 1) / PB;
-    const long long sstride = md_scratch_stride(P);
-    for (int a = 0; a < P.ndims; a++) {
-        const int nf = P.nmf[a];
-        const long long nfc = P.nb[a] / ((long long)nps * nf * 2);
-        const long long off = a == 0 ? 0 : (a == 1 ? (long long)P.ny * P.nz * nfm : ((long long)P.ny * P.nz + (long long)P.nx * P.nz) * nfm);
-        const long long offb = P.off_b[a];
-        const double *crow = P.cosv + (long long)a * nd;
-        const double *frow = P.frow_d + (long long)a * nd * nps;
-        const double *fex = P.fexit;
-        const long long nitem = nfc * nf * 2 * npb;
-        for (long long u = t.rank(); u < nitem; u += t.size()) {
-            const long long cell = u % nfc;
-            const long long rest = u / nfc;
-            const int is = (int)(rest % nf);
-            const int side = (int)((rest / nf) % 2);
-            const int p0 = (int)(rest / (2LL * nf)) * PB;
-            const double *ex = fex + off + cell * nfm + is;
-            double acc[PB];
-#pragma unroll
-            for (int q = 0; q < PB; q++) acc[q] = 0.0;
-            for (int n0 = 0; n0 < nd; n0 += 8) {
-                double v[8];
-                bool use[8];
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const int n = min(n0 + e, nd - 1);
-                    v[e] = ex[(long long)n * sstride];
-                    use[e] = n0 + e < nd && ((crow[n] >= 0.0) == (side == 1));
-                }
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const int n = min(n0 + e, nd - 1);
-                    const double *fr = frow + (long long)n * nps;
-#pragma unroll
-                    for (int q = 0; q < PB; q++) {
-                        const double w = fr[min(p0 + q, nps - 1)];
-                        acc[q] = fma(use[e] ? w : 0.0, v[e], acc[q]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < PB; q++) {
-                if (p0 + q >= nps) continue;
-                const long long k = offb + (p0 + q) + (long long)nps * (is + (long long)nf * (side + 2 * cell));
-                zout[k] = matvec ? zin[k] - acc[q] : acc[q];
-            }
-        }
-    }
-}
-
-// One thread per output, neighbouring lanes on neighbouring moments of one face cell (the exit
-// loads of a warp are one address): the layout for faces too small to give the blocked form
-// above a few items per thread.
+// over the directions leaving through that side (sn_sweep_2D.jl:146-179, accumulated over n as
+// sn_inner_pass.jl:127-129 does): for each face, side and face moment a product of the half-range
+// rows with the exits, on the FP64 tensor pipe. Per pass at 64³, S8: 200 us as sums over blocks of
+// moments per face cell; 2D, 128², S12: 50 us.
 template <class Team>
-__device__ void boundary_out_rows(Team &t, const DevProblem &P, const double *zin, double *zout, int matvec) {
-    const int nd = P.nd, nps = P.npsurf, nfm = P.nfmax;
+__device__ __noinline__ void boundary_out_md(Team &t, const DevProblem &P, void *region, long long bytes, const double *zin,
+                                             double *zout, int matvec) {
     const long long sstride = md_scratch_stride(P);
-    for (int a = 0; a < P.ndims; a++) {
+    const int nfm = P.nfmax, nps = P.npsurf, nd = P.nd;
+    if (nps == 0) return;
+    for_faces(t, P, [&](SubTeam st, int a, int side, int is) {
         const int nf = P.nmf[a];
         const long long off = a == 0 ? 0 : (a == 1 ? (long long)P.ny * P.nz * nfm : ((long long)P.ny * P.nz + (long long)P.nx * P.nz) * nfm);
-        for (long long o = t.rank(); o < P.nb[a]; o += t.size()) {
-            const int p = (int)(o % nps);
-            const int is = (int)((o / nps) % nf);
-            const int side = (int)((o / ((long long)nps * nf)) % 2);
-            const long long cell = o / ((long long)nps * nf * 2);
-            double s = 0.0;
-            for (int n = 0; n < nd; n++) {
-                const bool fwd = P.cosv[(long long)a * nd + n] >= 0.0;
-                if ((side == 1) == fwd)
-                    s += P.frow_d[((long long)a * nd + n) * nps + p] * P.fexit[(long long)n * sstride + off + cell * nfm + is];
-            }
-            const long long k = P.off_b[a] + o;
-            zout[k] = matvec ? zin[k] - s : s;
-        }
-    }
-}
-
-// Faces with many outputs per thread of the team take the blocked form with the largest moment
-// block that still gives every thread about two items; small faces take one thread per output.
-// Both forms give the same sums, in the same order.
-template <class Team>
-__device__ void boundary_out_md(Team &t, const DevProblem &P, const double *zin, double *zout, int matvec) {
-    long long outs = 0;
-    for (int a = 0; a < P.ndims; a++) outs += P.nb[a];
-    const long long want = 2LL * t.size();
-    if (outs / 16 >= want) boundary_out_pb<16>(t, P, zin, zout, matvec);
-    else if (outs / 4 >= want) boundary_out_pb<4>(t, P, zin, zout, matvec);
-    else boundary_out_rows(t, P, zin, zout, matvec);
+        const long long o0 = P.off_b[a] + (long long)nps * (is + (long long)nf * side);
+        Prod64 p{};
+        p.A = P.frow_d + (long long)a * nd * nps;
+        p.lda = nps;
+        p.ldi = 1;
+        p.ni = nps;
+        p.nk = nd;
+        p.X = P.fexit + off + is;
+        p.sx = sstride;
+        p.ldx = nfm;
+        p.ncol = P.fcells[a];
+        p.nm = 1;
+        p.pre = matvec ? zin + o0 : nullptr;
+        p.alpha = matvec ? -1.0 : 1.0;
+        p.out = zout + o0;
+        p.so = 1;
+        p.ldo = 2LL * nps * nf;
+        p.sel = P.cosv + (long long)a * nd;
+        p.selk = true;
+        p.selpos = side == 1;
+        prod64_team(st, p, region, bytes);
+    });
 }
 
 }  // namespace rb

@@ -12,15 +12,17 @@
 // memory. Every (octant batch, tile) is one task on one CTA of the team; a tile is paced by its
 // upwind tiles through per-CTA progress flags (a release after each pair of steps, an acquire
 // before the faces of a step are staged), so it runs about one tile height behind them with no
-// team barrier inside the sweep. The cell's inputs (angular source, material, incoming
-// energy-face flux, and the faces entering the tile) are staged one step ahead with cp.async.
+// team barrier inside the sweep. A step's cells are staged a step ahead with cp.async, each warp
+// its own 32 cells, and written back by the same lanes.
 // Each cell sees the same upwind faces as in the reference's lexicographic order
 // (sn_sweep_3D.jl:73-110), so the result equals it up to rounding.
 //
 // 2D: the KBA wavefront of sweep_md (rows of a direction skewed by one column per row, y faces
-// handed between rows through shared memory), one direction per thread, with the next cell's
-// inputs loaded one step ahead.
+// handed between rows through shared memory), one direction per thread, with the cells' inputs
+// loaded several steps ahead.
 #pragma once
+#include <type_traits>
+
 #include "rb_sweep_md.cuh"
 #include "rb_tc.cuh"
 
@@ -54,49 +56,56 @@ __device__ __forceinline__ bool one_moment_md(const DevProblem &P) {
     return P.nm5 == 1 && P.nmf[0] == 1 && P.nmf[1] == 1 && (P.ndims < 3 || P.nmf[2] == 1) && P.nm4 == 1;
 }
 
-template <typename R> struct OctDB { static constexpr int value = 10; };  // FP64: registers
+// Directions a thread solves per cell at the most: by its registers (FP64: fx, fy, the cell's and
+// the next cell's inputs are 20 registers each for 10 directions).
+template <typename R> struct OctDB { static constexpr int value = 10; };
 template <> struct OctDB<float> { static constexpr int value = 12; };
 
-// Stages of a step's inputs (cp.async, one step ahead): three, which lets a step write back the
-// previous step's flux after its single barrier; two for FP64 with CSD (three do not fit beside
-// the FP64 energy-face stages), with a second barrier per step.
-template <typename R, bool CSD> struct OctNB { static constexpr int value = 3; };
-template <> struct OctNB<double, true> { static constexpr int value = 2; };
 #define RB_OCT_MAXNX 1024  // x widths whose inverses the sweep keeps in shared memory
 #define RB_OCT_PUB 2       // a CTA publishes its progress every RB_OCT_PUB steps (and after its last)
+#define RB_OCT_PUBLISHER 128  // the thread that publishes
 
-// Shared-memory plan of the 3D octant sweep (byte offsets, each array 16-byte aligned): the
-// staged upwind faces of the tile's first row and layer of pencils, OctNB stages of a step's
-// angular source / flux, energy-face flux (CSD) and materials, the z-face hand-off between
-// pencils (double-buffered by step parity), the direction constants of the octant batch, the
-// inverse x widths and the per-material cell terms, and each pencil's cell base and coordinates.
-template <typename R, bool CSD>
+// Directions per octant batch: the octants are cut into as many batches as give every CTA of the
+// team a task in one round (a step's time is nearly proportional to its directions, its number of
+// steps is not), at least as many as the registers need, in even sizes (pair loads).
+__device__ __forceinline__ int oct_db(const DevProblem &P, int ncta, int ntiles, int dbmax) {
+    int cmax = 1;
+    for (int o = 0; o < P.noct; o++) cmax = max(cmax, P.oct_start[o + 1] - P.oct_start[o]);
+    const int need = (cmax + dbmax - 1) / dbmax, room = ncta / (ntiles * P.noct);
+    const int nb = max(need, min(room, (cmax + 1) / 2));
+    const int db = (cmax + nb - 1) / nb;
+    return min(dbmax, db > 1 ? (db + 1) & ~1 : 1);
+}
+
+// Shared-memory plan of the 3D octant sweep (byte offsets, each array 16-byte aligned): two stages
+// of the upwind faces of the tile's first row and layer of pencils and of every warp's cells
+// (angular source / flux and energy-face flux), the z-face hand-off between pencils
+// (double-buffered by step parity), the direction constants of the octant batch, the inverse x
+// widths, the per-material cell terms, and the materials of the tile's cells (a byte each, rows
+// padded so that a warp's 32 rows fall into different banks; longer pencils read them from memory).
+#define RB_OCT_MATNX 96  // longest pencil whose materials are kept in shared memory
+template <typename R>
 struct Oct3dSmem {
-    static constexpr long long DB = OctDB<R>::value, T = RB_OCT_TILE, TP = T * T, NB = OctNB<R, CSD>::value;
+    static constexpr long long DB = OctDB<R>::value, T = RB_OCT_TILE, TP = T * T;
     static constexpr long long RS = (long long)sizeof(R);
+    static constexpr int DC = sizeof(R) == 8 ? 10 : 12;                      // constants per direction, padded to 16 bytes
+    static constexpr long long CS = DB % 4 == 2 ? DB : DB + 2;               // widest cell stride of a stage (below)
+    static constexpr int MROW = RB_OCT_MATNX + 4;                            // bytes of a pencil's materials
     static constexpr long long al(long long b) { return (b + 15) & ~15LL; }
-    static constexpr long long fy = 0;                                      // double [NB][T][DB]
-    static constexpr long long fz = fy + al(NB * T * DB * 8);               // double [NB][T][DB]
-    static constexpr long long eb = fz + al(NB * T * DB * 8);               // double [NB][TP][DB]
-    static constexpr long long pcb = eb + (CSD ? al(NB * TP * DB * 8) : 0); // long long [TP]
-    static constexpr long long dc = pcb + al(TP * 8);                       // R [DB][9]
-    static constexpr long long sfz = dc + al(DB * 9 * RS);                  // R [2][DB][TP]
-    static constexpr long long qb = sfz + al(2 * DB * TP * RS);             // R [NB][TP][DB]
-    static constexpr long long ix = qb + al(NB * TP * DB * RS);             // R [RB_OCT_MAXNX]
+    static constexpr long long fy = 0;                                      // double [2][T][DB]
+    static constexpr long long fz = fy + al(2 * T * DB * 8);                // double [2][T][DB]
+    static constexpr long long dc = fz + al(2 * T * DB * 8);                // R [DB][DC]
+    static constexpr long long sfz = dc + al(DB * DC * RS);                 // R [2][DB][TP]
+    static constexpr long long qb = sfz + al(2 * DB * TP * RS);             // R [2][TP][CS]
+    static constexpr long long ix = qb + al(2 * CS * TP * RS);              // R [RB_OCT_MAXNX]
     static constexpr long long ms = ix + al(RB_OCT_MAXNX * RS);             // R [RB_MAXMAT]
     static constexpr long long mq = ms + al(RB_MAXMAT * RS);                // R [RB_MAXMAT]
-    static constexpr long long mb = mq + al(RB_MAXMAT * RS);                // int [NB][TP]
-    static constexpr long long pj = mb + al(NB * TP * 4);                   // int [TP]
-    static constexpr long long py = pj + al(TP * 4);                        // int [TP]
-    static constexpr long long pz = py + al(TP * 4);                        // int [TP]
-    static constexpr long long bytes = pz + al(TP * 4);
+    static constexpr long long mt = mq + al(RB_MAXMAT * RS);                // byte [TP][MROW]
+    static constexpr long long eb = mt + al(TP * MROW);                     // double [2][TP][CS] (CSD)
+    static constexpr long long bytes(bool csd) { return eb + (csd ? al(2 * CS * TP * 8) : 0); }
 };
-template <typename R, bool CSD>
-__host__ __device__ constexpr long long oct3d_smem() { return Oct3dSmem<R, CSD>::bytes; }
-__host__ __device__ constexpr long long oct3d_smem_max() {
-    return oct3d_smem<double, true>() > oct3d_smem<float, true>() ? oct3d_smem<double, true>()
-                                                                  : oct3d_smem<float, true>();
-}
+template <typename R>
+__host__ __device__ constexpr long long oct3d_smem(bool csd) { return Oct3dSmem<R>::bytes(csd); }
 
 // Tile height in y: a power of two up to RB_OCT_TILE, so that a pencil's lower neighbour is the
 // previous lane of the same warp.
@@ -110,11 +119,10 @@ __device__ __forceinline__ int oct_ty(int ny) {
 // CTA of the team has a progress flag, and the step and round counts fit their bit fields.
 __device__ __forceinline__ bool oct3d_ok(const DevProblem &P, int ncta, long long smem_bytes, int mixed) {
     if (P.ndims != 3 || !one_moment_md(P) || ncta > RB_OCT_MAXCTA) return false;
-    if (P.nx + 2 * RB_OCT_TILE >= (1 << 20) || P.nd >= (1 << 12)) return false;
+    if (P.nx + 2 * RB_OCT_TILE >= (1 << 20) || P.nd >= (1 << 12) || (long long)P.nd * P.ncell >= (1LL << 32)) return false;
     const int TY = oct_ty(P.ny), TZ = min(P.nz, RB_OCT_TILE);
     const int ntiles = ((P.ny + TY - 1) / TY) * ((P.nz + TZ - 1) / TZ);
-    const long long need = mixed ? (P.csd ? oct3d_smem<float, true>() : oct3d_smem<float, false>())
-                                 : (P.csd ? oct3d_smem<double, true>() : oct3d_smem<double, false>());
+    const long long need = mixed ? oct3d_smem<float>(P.csd) : oct3d_smem<double>(P.csd);
     return ntiles <= ncta && smem_bytes >= need;
 }
 
@@ -151,10 +159,27 @@ __device__ __forceinline__ bool wait_progress(const unsigned long long *f, unsig
     return false;
 }
 
-// q / S of a cell: IEEE division in FP64 (the plain form), the fast reciprocal-based division
-// in FP32 (the mixed form, whose FP64 defect correction absorbs its 2-ulp error)
-__device__ __forceinline__ double oct_div(double q, double s) { return q / s; }
+// q / S of a cell. FP32 (mixed form): the fast reciprocal-based division, whose 2-ulp error the
+// FP64 defect correction absorbs. FP64 (plain form): the correctly rounded quotient by Newton's
+// reciprocal and Markstein's final correction (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990) without a branch, so the chains of a cell's
+// directions interleave; the divide instruction sequence ends each one in a branch. Operands
+// outside the range where the correction is exact take the divide.
+__device__ __forceinline__ double oct_div(double q, double s) {
+    const double a = fabs(s);
+    if (!(a > 1e-140 && a < 1e140)) return q / s;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
+    r = fma(r, fma(-s, r, 1.0), r);
+    r = fma(r, fma(-s, r, 1.0), r);
+    const double v = q * r;
+    return fma(fma(-s, v, q), r, v);
+}
 __device__ __forceinline__ float oct_div(float q, float s) { return __fdividef(q, s); }
+
+template <typename T> struct Pair;
+template <> struct Pair<float> { using type = float2; };
+template <> struct Pair<double> { using type = double2; };
 
 // The sweep of one octant batch over one tile of pencils is a task; the tasks of a round (one per
 // CTA) run concurrently, and a tile is paced by the tiles upwind of it in y and z: before it
@@ -163,20 +188,24 @@ __device__ __forceinline__ float oct_div(float q, float s) { return __fdividef(q
 // it has completed, tagged with the sweep's epoch and the round, after a barrier that follows the
 // face stores and a GPU-scope fence, so a downstream tile runs about TY steps behind its upwind
 // tile with no team barrier inside the sweep.
-template <typename R, typename PS, bool CSD, class Team>
-__device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShared &gs, void *smem, const double *zin,
-                                         int np_source, const double *phiE_in, double *phiE_out, int ig, PS *psi) {
-    using L = Oct3dSmem<R, CSD>;
-    static_assert(sizeof(PS) == sizeof(R), "angular buffer and arithmetic of one width");
-    constexpr int DB = OctDB<R>::value, TT = RB_OCT_TILE, TP = TT * TT, NB = OctNB<R, CSD>::value;
-    // one barrier per step: the write-back and the publication of step sg follow the barrier of
-    // step sg + 1, which also orders the z-face hand-off; the stage being written back is then
-    // neither the one being staged nor the one being solved
-    constexpr bool ONEBAR = NB >= 3;
+//
+// What bounds it: the L1 line lookups of a step (about two cycles each) and the chain barrier,
+// faces, cells, barrier. A lane that reads its own cell's directions touches a line per lane and
+// load, so a warp's 32 cells are staged together, cnt / VW neighbouring lanes on the run of one
+// cell, with each lane's pencils and offsets worked out once per task; the same lanes write the
+// results back. VW = 2: the batch's directions start and count even (pairs). Sweep at 64³, S8,
+// mixed: 2070 us (element-wise staging, addresses per element), 1030 (each thread its own cell).
+// RECIP: the cell as sweep_3d_tiles solves it (DevProblem::recip).
+template <typename R, int DB, int VW, bool CSD, bool RECIP, class Team>
+__device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShared &gs, void *smem,
+                                         const double *phiE_in, double *phiE_out, R *psi, int db) {
+    using L = Oct3dSmem<R>;
+    constexpr int TT = RB_OCT_TILE, TP = TT * TT, DC = L::DC, LDB = OctDB<R>::value;
+    constexpr int CS = DB % 4 == 2 ? DB : DB + 2;  // cell stride of a stage: pair loads of a warp free of bank conflicts
     const int nd = P.nd, nx = P.nx, ny = P.ny, nz = P.nz, nfm = P.nfmax;
     const int TY = oct_ty(ny), TZ = min(nz, RB_OCT_TILE);
     const int nty = (ny + TY - 1) / TY, ntz = (nz + TZ - 1) / TZ, ntiles = nty * ntz;
-    const int ngrp = oct_groups(P, DB);
+    const int ngrp = oct_groups(P, db);
     const int gpr = (int)t.ncta / ntiles;  // octant batches per round (≥ 1: oct3d_ok)
     const int nround = (ngrp + gpr - 1) / gpr;
     const int nsteps = nx + TY + TZ - 2;
@@ -190,19 +219,15 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
     unsigned char *base = reinterpret_cast<unsigned char *>(smem);
     double *fyb = reinterpret_cast<double *>(base + L::fy);
     double *fzb = reinterpret_cast<double *>(base + L::fz);
-    double *eb = reinterpret_cast<double *>(base + L::eb);
-    long long *pcb = reinterpret_cast<long long *>(base + L::pcb);
     R *dc = reinterpret_cast<R *>(base + L::dc);
     R *sfz = reinterpret_cast<R *>(base + L::sfz);
-    PS *qb = reinterpret_cast<PS *>(base + L::qb);
     R *idxs = reinterpret_cast<R *>(base + L::ix);
     R *mS = reinterpret_cast<R *>(base + L::ms);
     R *mQ = reinterpret_cast<R *>(base + L::mq);
-    int *mb = reinterpret_cast<int *>(base + L::mb);
-    int *pjs = reinterpret_cast<int *>(base + L::pj);
-    int *piy = reinterpret_cast<int *>(base + L::py);
-    int *piz = reinterpret_cast<int *>(base + L::pz);
-    const int me = threadIdx.x, jy = me % TY, jz = me / TY;
+    unsigned char *mt = base + L::mt;
+    const int me = threadIdx.x, lane = me & 31, jy = me % TY, jz = me / TY;
+    R *qb = reinterpret_cast<R *>(base + L::qb) + (me - lane) * CS;                       // this warp's [32][CS]
+    double *eb = reinterpret_cast<double *>(base + L::eb) + (CSD ? (me - lane) * CS : 0);  // (stages TP·CS apart)
     const R w1x = (R)P.w1[0], w1y = (R)P.w1[1], w1z = (R)P.w1[2], w1e = (R)P.w1[3];
     const R esa = CSD ? (R)P.EsA[0] : R(0), esb = CSD ? (R)P.EsB[0] : R(0), eout = CSD ? (R)P.Eout[0] : R(0);
     // this sweep's tables: inverse x widths, and per material Σt (+ the CSD cell term) and the
@@ -226,51 +251,65 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
     const unsigned long long epoch = (unsigned long long)gs.oct_epoch;
     unsigned long long seen_y = 0, seen_z = 0;  // thread 0: the upwind flags as last read
     bool gave_up = false;
+    const int *mat = P.mat;
+    double *fexit = P.fexit;
+    unsigned long long *flags = P.oct_flags;
     for (int rnd = 0; rnd < nround; rnd++) {
         const int g = rnd * gpr + (int)t.crank / ntiles;
         const int tile = (int)t.crank % ntiles;
         int first = 0, cnt = 0, oc = 0;
-        if ((int)t.crank < gpr * ntiles && g < ngrp) oc = oct_group(P, DB, g, first, cnt);
+        if ((int)t.crank < gpr * ntiles && g < ngrp) oc = oct_group(P, db, g, first, cnt);
         if (cnt == 0) continue;  // uniform over the CTA
         const bool fx = !(oc & 1), fy = !(oc & 2), fz = !(oc & 4);
+        const int parts = cnt / VW;
         const int tyq = tile % nty, tzq = tile / nty;  // tile coordinates in sweep order
         const int iyy = tyq * TY + jy, izz = tzq * TZ + jz;
         const bool pok = me < TY * TZ && iyy < ny && izz < nz;
         const int iy = fy ? iyy : ny - 1 - iyy, iz = fz ? izz : nz - 1 - izz;
         const unsigned long long tagr = (epoch << 32) | ((unsigned long long)rnd << 20);
-        const unsigned long long *upy = tyq > 0 ? P.oct_flags + (t.crank - 1) : nullptr;
-        const unsigned long long *upz = tzq > 0 ? P.oct_flags + (t.crank - nty) : nullptr;
+        const unsigned long long *upy = tyq > 0 ? flags + (t.crank - 1) : nullptr;
+        const unsigned long long *upz = tzq > 0 ? flags + (t.crank - nty) : nullptr;
         __syncthreads();  // the previous round's readers of the region are done
-        if (me < DB) {
+        if (me < LDB) {
             const int n = first + me;
             for (int a = 0; a < 3; a++) {
                 const long long blk = (long long)n * 3 + a;
-                const double ac = me < cnt ? fabs(P.cosv[(long long)a * nd + n]) : 0.0;
-                dc[me * 9 + a] = me < cnt ? (R)(ac * P.G[blk]) : R(0);
-                dc[me * 9 + 3 + a] = me < cnt ? (R)(ac * P.Gsrc[blk * nfm]) : R(0);
-                dc[me * 9 + 6 + a] = me < cnt ? (R)P.Gout[blk * nfm] : R(0);
+                const double ac = RECIP ? 1.0 : (me < cnt ? fabs(P.cosv[(long long)a * nd + n]) : 0.0);
+                dc[me * DC + a] = me < cnt ? (R)(ac * P.G[blk]) : R(0);
+                dc[me * DC + 3 + a] = me < cnt ? (R)(ac * P.Gsrc[blk * nfm]) : R(0);
+                dc[me * DC + 6 + a] = me < cnt ? (R)P.Gout[blk * nfm] : R(0);
             }
         }
-        if (me < TP) {
-            pcb[me] = pok ? (long long)nx * (iy + (long long)ny * iz) : -1;
-            pjs[me] = jy + jz;
-            piy[me] = iy;
-            piz[me] = iz;
+        // The faces entering the tile in a step, one direction of one pencil per item: pencils
+        // (0, j) for y faces, then (j, 0) for z faces; a thread has up to RB_OCT_ITEMS of them.
+        constexpr int NI = (2 * TT * DB + TP - 1) / TP;
+        const double *isrc[NI];  // the item's face at x column 0
+        int ij[NI], idst[NI];    // its pencil's offset in steps (−1: none) and place in a stage
+        {
+            const int nfy = TZ * cnt, nfz = TY * cnt;
+#pragma unroll
+            for (int u = 0; u < NI; u++) {
+                const int e = me + u * TP;
+                ij[u] = -1;
+                isrc[u] = nullptr;
+                idst[u] = 0;
+                if (e < nfy + nfz) {
+                    const bool isy = e < nfy;
+                    const int e2 = isy ? e : e - nfy, j = e2 / cnt, kk = e2 - j * cnt;
+                    const int qy = tyq * TY + (isy ? 0 : j), qz = tzq * TZ + (isy ? j : 0);
+                    if (qy < ny && qz < nz) {
+                        const int row = isy ? (fz ? qz : nz - 1 - qz) : (fy ? qy : ny - 1 - qy);
+                        const long long off = isy ? (tyq == 0 ? yin : yoff) : (tzq == 0 ? zin_ : zoff);
+                        isrc[u] = fexit + (long long)(first + kk) * sstride + off + (long long)nx * row * nfm;
+                        ij[u] = j;
+                        idst[u] = (isy ? 0 : (int)((L::fz - L::fy) / 8)) + j * LDB + kk;
+                    }
+                }
+            }
         }
-        __syncthreads();
-        // A step's cells are staged cooperatively: element e = me + TP·r (r < cnt) of the step is
-        // direction k = e % cnt of pencil p = e / cnt, so consecutive lanes read consecutive
-        // directions of a cell (one contiguous run of cnt values per cell).
-        const int qd = TP / cnt, rm = TP % cnt, p0 = me / cnt, k0 = me % cnt;
-        auto cell_of = [&](int p, int sg) -> long long {  // cell of pencil p at step sg, −1 if none
-            const long long cb = pcb[p];
-            const int ixx = sg - pjs[p];
-            if (cb < 0 || ixx < 0 || ixx >= nx) return -1;
-            return cb + (fx ? ixx : nx - 1 - ixx);
-        };
         // thread 0: the upwind tiles have published the steps that write the faces of step s
         auto wait_up = [&](int s) {
-            if (me != 0 || gave_up || s < 0 || s >= nsteps) return;
+            if (me != 0 || gave_up || s >= nsteps) return;
             bool ok = true;
             if (upy) ok = wait_progress(upy, tagr | (unsigned long long)(min(s + TY - 1, nsteps - 1) + 1), seen_y);
             if (ok && upz) ok = wait_progress(upz, tagr | (unsigned long long)(min(s + TZ - 1, nsteps - 1) + 1), seen_z);
@@ -279,278 +318,701 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                 atomicOr(P.status, RB_DEV_TIMEOUT);
             }
         };
-        // step s's inputs into stage s % NB (one commit group): angular source, energy-face flux,
-        // materials, and the faces entering the tile's pencils (0, jz) and (jy, 0)
-        auto issue = [&](int s) {
-            if (s >= 0 && s < nsteps) {
-                const int st = s % NB;
-                int p = p0, k = k0;
+        auto stage_faces = [&](int s) {
+            if (s < nsteps) {
 #pragma unroll
-                for (int r = 0; r < DB; r++) {
-                    if (r < cnt) {
-                        const long long c = cell_of(p, s);
-                        if (c >= 0) {
-                            const long long so = ((long long)st * TP + p) * DB + k;
-                            const long long go = first + k + (long long)nd * c;
-                            cp_async<sizeof(PS)>(qb + so, psi + go);
-                            if (CSD && phiE_in) cp_async<8>(eb + so, phiE_in + go);
-                        }
-                    }
-                    p += qd;
-                    k += rm;
-                    if (k >= cnt) { k -= cnt; p++; }
-                }
-                {
-                    const long long c = cell_of(me, s);
-                    if (c >= 0) cp_async<4>(mb + st * TP + me, P.mat + c);
-                }
-                const int nfy = TZ * cnt, nfz = TY * cnt;
-                for (int e = me; e < nfy + nfz; e += blockDim.x) {
-                    const bool isy = e < nfy;
-                    const int e2 = isy ? e : e - nfy;
-                    const int j = e2 / cnt, kk = e2 % cnt;  // pencil (0, j) for y faces, (j, 0) for z faces
-                    const int pp = isy ? TY * j : j;
-                    const int ixx = s - j;
-                    if (pcb[pp] >= 0 && ixx >= 0 && ixx < nx) {
-                        const int ix = fx ? ixx : nx - 1 - ixx;
-                        const long long o = isy ? (tyq == 0 ? yin : yoff) + (ix + (long long)nx * piz[pp]) * nfm
-                                                : (tzq == 0 ? zin_ : zoff) + (ix + (long long)nx * piy[pp]) * nfm;
-                        cp_async<8>((isy ? fyb : fzb) + ((long long)st * TT + j) * DB + kk,
-                                    P.fexit + (long long)(first + kk) * sstride + o);
-                    }
+                for (int u = 0; u < NI; u++) {
+                    const int ixx = s - ij[u];
+                    if (ij[u] >= 0 && ixx >= 0 && ixx < nx)
+                        cp_async<8>(fyb + (s & 1) * (TT * LDB) + idst[u], isrc[u] + (long long)(fx ? ixx : nx - 1 - ixx) * nfm);
                 }
             }
             cp_async_commit();
         };
         const R idy = pok ? (R)(1.0 / P.dy[iy]) : R(0), idz = pok ? (R)(1.0 / P.dz[iz]) : R(0);
+        const unsigned c0 = (unsigned)nx * (iy + ny * iz);  // the pencil's first cell
+        const int dstep = jy + jz;                          // the pencil's first step
+        // element e = lane + 32·i of the warp's cells: part e % parts of pencil e / parts: its offset
+        // in ψ at x column −(steps it runs behind), its steps behind, its place in a stage
+        constexpr int NE = DB / VW;
+        unsigned eo[NE];
+        int ed[NE], ep[NE];
+        const unsigned estep = fx ? (unsigned)nd : 0u - (unsigned)nd;  // a column further
+#pragma unroll
+        for (int i = 0; i < NE; i++) {
+            const int e = lane + 32 * i, pl = e / parts, part = e - pl * parts;
+            const int pm = (me - lane) + (pl < 32 ? pl : 0), py = pm % TY, pz = pm / TY;
+            const int qy = tyq * TY + py, qz = tzq * TZ + pz;
+            const bool ok = i < parts && pm < TY * TZ && qy < ny && qz < nz;
+            ed[i] = ok ? py + pz : 1 << 28;
+            ep[i] = pl * CS + part * VW;
+            const unsigned row = (unsigned)nx * ((fy ? qy : ny - 1 - qy) + ny * (fz ? qz : nz - 1 - qz));
+            eo[i] = ok ? (unsigned)nd * (row + (fx ? 0 : nx - 1)) + first + part * VW - (unsigned)ed[i] * estep : 0;
+        }
+        // the warp's cells of step s into stage s & 1
+        auto stage_cells = [&](int s) {
+            const int st = (s & 1) * (TP * CS);
+#pragma unroll
+            for (int i = 0; i < NE; i++) {
+                if (i < parts && (unsigned)(s - ed[i]) < (unsigned)nx) {
+                    const unsigned o = eo[i] + (unsigned)s * estep;
+                    cp_async<VW * (int)sizeof(R)>(qb + st + ep[i], psi + o);
+                    if (CSD && phiE_in) cp_async<VW * 8>(eb + st + ep[i], phiE_in + o);
+                }
+            }
+        };
+        auto store_cells = [&](int s) {
+            const int st = (s & 1) * (TP * CS);
+#pragma unroll
+            for (int i = 0; i < NE; i++) {
+                if (i < parts && (unsigned)(s - ed[i]) < (unsigned)nx) {
+                    const unsigned o = eo[i] + (unsigned)s * estep;
+                    if constexpr (VW == 2) {
+                        using R2 = typename Pair<R>::type;
+                        *reinterpret_cast<R2 *>(psi + o) = *reinterpret_cast<const R2 *>(qb + st + ep[i]);
+                        if (CSD && phiE_out)
+                            *reinterpret_cast<double2 *>(phiE_out + o) = *reinterpret_cast<const double2 *>(eb + st + ep[i]);
+                    } else {
+                        psi[o] = qb[st + ep[i]];
+                        if (CSD && phiE_out) phiE_out[o] = eb[st + ep[i]];
+                    }
+                }
+            }
+        };
+        const bool mat_sm = nx <= RB_OCT_MATNX;
+        if (mat_sm)  // materials of the tile's pencils, a row per warp
+            for (int p = me >> 5; p < TP; p += RB_THREADS / 32) {
+                const int qy = tyq * TY + p % TY, qz = tzq * TZ + p / TY;
+                if (p < TY * TZ && qy < ny && qz < nz) {
+                    const int *m = mat + (long long)nx * ((fy ? qy : ny - 1 - qy) + ny * (fz ? qz : nz - 1 - qz));
+                    for (int x = lane; x < nx; x += 32) mt[p * L::MROW + x] = (unsigned char)m[x];
+                }
+            }
         R fxs[DB], fyl[DB];
         {
             const long long o = xin + (iy + (long long)ny * iz) * nfm;  // the domain's incoming x faces
 #pragma unroll
             for (int k = 0; k < DB; k++) {
                 fyl[k] = R(0);
-                fxs[k] = (pok && k < cnt) ? (R)P.fexit[(long long)(first + k) * sstride + o] : R(0);
+                fxs[k] = (pok && k < cnt) ? (R)fexit[(long long)(first + k) * sstride + o] : R(0);
             }
         }
-        // step s done by every thread: publish it (the barrier before this orders every thread's
-        // face stores before thread 0's fence and release), then write its stage back, consecutive
-        // lanes on consecutive directions of a cell
-        auto finish = [&](int s) {
-            if (me == 0 && ((s + 1) % RB_OCT_PUB == 0 || s == nsteps - 1)) {
-                __threadfence();
-                st_release_u64(P.oct_flags + t.crank, tagr | (unsigned long long)(s + 1));
-            }
-            const int ss = s % NB;
-            int p = p0, k = k0;
-#pragma unroll
-            for (int r = 0; r < DB; r++) {
-                if (r < cnt) {
-                    const long long c = cell_of(p, s);
-                    if (c >= 0) {
-                        const long long so = ((long long)ss * TP + p) * DB + k;
-                        const long long go = first + k + (long long)nd * c;
-                        psi[go] = qb[so];
-                        if (CSD) phiE_out[go] = eb[so];
-                    }
-                }
-                p += qd;
-                k += rm;
-                if (k >= cnt) { k -= cnt; p++; }
-            }
-        };
         wait_up(0);
         __syncthreads();
-        issue(0);
+        stage_cells(0);
+        stage_faces(0);
         for (int sg = 0; sg < nsteps; sg++) {
             wait_up(sg + 1);
             cp_async_wait<0>();  // this thread's copies of step sg have landed
             __syncthreads();     // everyone's; step sg − 1 solved; step sg + 1's faces are written
-            if (ONEBAR && sg > 0) finish(sg - 1);
-            issue(sg + 1);       // in flight while step sg is solved
-            const int ixx = sg - jy - jz;
-            const int rd = (sg + 1) & 1, wr = sg & 1, sb = sg % NB;
+            // steps < sg are done: publish (the barrier orders every thread's face stores before the
+            // release), by another warp than the one that waits for the upwind tiles
+            if (me == RB_OCT_PUBLISHER && sg > 0 && sg % RB_OCT_PUB == 0)
+                st_release_u64(flags + t.crank, tagr | (unsigned long long)sg);
+            if (sg + 1 < nsteps) stage_cells(sg + 1);
+            stage_faces(sg + 1);
+            const int ixx = sg - dstep;
+            const int rd = (sg + 1) & 1, wr = sg & 1;
             R fyi[DB];
 #pragma unroll
             for (int k = 0; k < DB; k++) fyi[k] = __shfl_up_sync(0xffffffffu, fyl[k], 1);
             if (pok && ixx >= 0 && ixx < nx) {
                 const int ix = fx ? ixx : nx - 1 - ixx;
-                const long long yk = (ix + (long long)nx * iz) * nfm, zk = (ix + (long long)nx * iy) * nfm;
-                // every input of the cell first, then the arithmetic, then the stores (no shared
-                // store sits between two loads, so the directions' chains overlap)
-                R fzi[DB], qv[DB], fe[DB];
-                PS *qc = qb + ((long long)sb * TP + me) * DB;
-                double *ec = eb + ((long long)sb * TP + me) * DB;
+                R fzi[DB];
+                R *qc = qb + wr * (TP * CS) + lane * CS;
+                double *ec = eb + wr * (TP * CS) + lane * CS;
                 if (jy == 0) {
 #pragma unroll
-                    for (int k = 0; k < DB; k++) fyi[k] = (R)fyb[((long long)sb * TT + jz) * DB + k];
+                    for (int k = 0; k < DB; k++) fyi[k] = (R)fyb[(wr * TT + jz) * LDB + k];
                 }
                 if (jz == 0) {
 #pragma unroll
-                    for (int k = 0; k < DB; k++) fzi[k] = (R)fzb[((long long)sb * TT + jy) * DB + k];
+                    for (int k = 0; k < DB; k++) fzi[k] = (R)fzb[(wr * TT + jy) * LDB + k];
                 } else {
 #pragma unroll
-                    for (int k = 0; k < DB; k++) fzi[k] = sfz[(rd * DB + k) * TP + me - TY];
+                    for (int k = 0; k < DB; k++) fzi[k] = sfz[(rd * LDB + k) * TP + me - TY];
                 }
+                R v[DB], fe[CSD ? DB : 1];
+                if constexpr (VW == 2) {
 #pragma unroll
-                for (int k = 0; k < DB; k++) {
-                    qv[k] = (R)qc[k];
-                    fe[k] = (CSD && phiE_in) ? (R)ec[k] : R(0);
+                    for (int k = 0; k < DB; k += 2) {
+                        const auto x = *reinterpret_cast<const typename Pair<R>::type *>(qc + k);
+                        v[k] = x.x;
+                        v[k + 1] = x.y;
+                        if constexpr (CSD) {
+                            double2 e = make_double2(0.0, 0.0);
+                            if (phiE_in) e = *reinterpret_cast<const double2 *>(ec + k);
+                            fe[k] = (R)e.x;
+                            fe[k + 1] = (R)e.y;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < DB; k++) {
+                        v[k] = qc[k];
+                        if (CSD) fe[CSD ? k : 0] = phiE_in ? (R)ec[k] : R(0);
+                    }
                 }
-                const int m = mb[sb * TP + me];
+                const int m = mat_sm ? mt[me * L::MROW + ix] : mat[c0 + ix];
                 const R S0 = mS[m], sq = mQ[m];
                 const R idx = xs_sm ? idxs[ix] : (R)(1.0 / P.dx[ix]);
-                R v[DB];
+                if constexpr (RECIP) {
 #pragma unroll
-                for (int k = 0; k < DB; k++) {
-                    const R *d = dc + k * 9;
-                    const R S = S0 + d[0] * idx + d[1] * idy + d[2] * idz;
-                    R q = qv[k] + (d[3] * idx) * fxs[k] + (d[4] * idy) * fyi[k] + (d[5] * idz) * fzi[k];
-                    if (CSD) q -= sq * fe[k];
-                    v[k] = oct_div(q, S);
-                    fxs[k] = w1x * fxs[k] + d[6] * v[k];
-                    fyi[k] = w1y * fyi[k] + d[7] * v[k];
-                    fzi[k] = w1z * fzi[k] + d[8] * v[k];
+                    for (int k = 0; k < DB; k++) {
+                        if (k >= cnt) continue;
+                        const R *d = dc + k * DC;
+                        const int n = first + k;
+                        const R hx = oct_div(fabs(P.cosv[n]), P.dx[ix]), hy = oct_div(fabs(P.cosv[nd + n]), P.dy[iy]);
+                        const R hz = oct_div(fabs(P.cosv[2 * nd + n]), P.dz[iz]);
+                        R S = S0, q = v[k];
+                        S += hx * d[0];
+                        S += hy * d[1];
+                        S += hz * d[2];
+                        q += hx * (d[3] * fxs[k]);
+                        q += hy * (d[4] * fyi[k]);
+                        q += hz * (d[5] * fzi[k]);
+                        v[k] = q * oct_div(1.0, S);
+                        fxs[k] = w1x * fxs[k] + d[6] * v[k];
+                        fyi[k] = w1y * fyi[k] + d[7] * v[k];
+                        fzi[k] = w1z * fzi[k] + d[8] * v[k];
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < DB; k++) {
+                        const R *d = dc + k * DC;
+                        const R S = S0 + d[0] * idx + d[1] * idy + d[2] * idz;
+                        R q = v[k] + (d[3] * idx) * fxs[k] + (d[4] * idy) * fyi[k] + (d[5] * idz) * fzi[k];
+                        if (CSD) q -= sq * fe[CSD ? k : 0];
+                        v[k] = oct_div(q, S);
+                        fxs[k] = w1x * fxs[k] + d[6] * v[k];
+                        fyi[k] = w1y * fyi[k] + d[7] * v[k];
+                        fzi[k] = w1z * fzi[k] + d[8] * v[k];
+                    }
                 }
 #pragma unroll
-                for (int k = 0; k < DB; k++) {
-                    if (k >= cnt) continue;
-                    qc[k] = (PS)v[k];
-                    if (CSD) ec[k] = (double)(w1e * fe[k] + eout * v[k]);
-                    sfz[(wr * DB + k) * TP + me] = fzi[k];
+                for (int k = 0; k < DB; k++)
+                    if (k < cnt) sfz[(wr * LDB + k) * TP + me] = fzi[k];
+                if constexpr (VW == 2) {
+#pragma unroll
+                    for (int k = 0; k < DB; k += 2) {
+                        typename Pair<R>::type x;
+                        x.x = v[k];
+                        x.y = v[k + 1];
+                        *reinterpret_cast<typename Pair<R>::type *>(qc + k) = x;
+                        if (CSD && phiE_out)
+                            *reinterpret_cast<double2 *>(ec + k) =
+                                make_double2((double)(w1e * fe[CSD ? k : 0] + eout * v[k]), (double)(w1e * fe[CSD ? k + 1 : 0] + eout * v[k + 1]));
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < DB; k++) {
+                        qc[k] = v[k];
+                        if (CSD) ec[k] = (double)(w1e * fe[CSD ? k : 0] + eout * v[k]);
+                    }
                 }
                 // faces leaving the tile or the domain
                 if (jy == TY - 1 || iyy == ny - 1) {
-                    const long long off = iyy < ny - 1 ? yoff : eyo;
+                    double *f = fexit + (long long)first * sstride + (iyy < ny - 1 ? yoff : eyo) + (ix + (long long)nx * iz) * nfm;
 #pragma unroll
                     for (int k = 0; k < DB; k++)
-                        if (k < cnt) P.fexit[(long long)(first + k) * sstride + off + yk] = (double)fyi[k];
+                        if (k < cnt) f[(long long)k * sstride] = (double)fyi[k];
                 }
                 if (jz == TZ - 1 || izz == nz - 1) {
-                    const long long off = izz < nz - 1 ? zoff : ezo;
+                    double *f = fexit + (long long)first * sstride + (izz < nz - 1 ? zoff : ezo) + (ix + (long long)nx * iy) * nfm;
 #pragma unroll
                     for (int k = 0; k < DB; k++)
-                        if (k < cnt) P.fexit[(long long)(first + k) * sstride + off + zk] = (double)fzi[k];
+                        if (k < cnt) f[(long long)k * sstride] = (double)fzi[k];
                 }
                 if (ixx == nx - 1) {
-                    const long long o = (iy + (long long)ny * iz) * nfm;
+                    double *f = fexit + (long long)first * sstride + (iy + (long long)ny * iz) * nfm;
 #pragma unroll
                     for (int k = 0; k < DB; k++)
-                        if (k < cnt) P.fexit[(long long)(first + k) * sstride + o] = (double)fxs[k];
+                        if (k < cnt) f[(long long)k * sstride] = (double)fxs[k];
                 }
             }
 #pragma unroll
             for (int k = 0; k < DB; k++) fyl[k] = fyi[k];
-            if (!ONEBAR) {
-                __syncthreads();
-                finish(sg);
-            }
-        }
-        if (ONEBAR && nsteps > 0) {
-            __syncthreads();
-            finish(nsteps - 1);
+            __syncwarp();
+            store_cells(sg);
+            __syncwarp();  // before the stage takes the step after the next
         }
         cp_async_wait<0>();
         __syncthreads();
+        if (me == RB_OCT_PUBLISHER) st_release_u64(flags + t.crank, tagr | (unsigned long long)nsteps);
     }
+    __syncthreads();
 }
 
-// 2D, one-moment cells: sweep_md's wavefront with the next cell's inputs loaded one step ahead
-// and the arithmetic in R (FP64 or FP32) over an angular buffer of PS.
-template <typename R, typename PS, bool CSD, class Team>
-__device__ __noinline__ void sweep2d_pf(Team &t, const DevProblem &P, GroupShared &gs, const double *zin, int np_source,
-                           const double *phiE_in, double *phiE_out, int ig, PS *psi) {
-    const int nd = P.nd, nx = P.nx, ny = P.ny, nfm = P.nfmax;
+// the octant sweep with the smallest instantiated batch that holds the problem's
+template <typename R, bool CSD, class Team>
+__device__ __forceinline__ void sweep3d_run(Team &t, const DevProblem &P, GroupShared &gs, void *smem,
+                                            const double *phiE_in, double *phiE_out, R *psi) {
+    const int TY = oct_ty(P.ny), TZ = min(P.nz, RB_OCT_TILE);
+    const int db = oct_db(P, (int)t.ncta, ((P.ny + TY - 1) / TY) * ((P.nz + TZ - 1) / TZ), OctDB<R>::value);
+    // pairs: every octant starts even and has an even count, and so do its batches
+    bool even = P.nd % 2 == 0 && db % 2 == 0;
+    for (int o = 0; o < P.noct; o++) even = even && (P.oct_start[o + 1] - P.oct_start[o]) % 2 == 0;
+#define RB_OCT_RUN(DB_)                                                                                     \
+    {                                                                                                       \
+        if (even) sweep3d_oct<R, DB_, 2, CSD, false>(t, P, gs, smem, phiE_in, phiE_out, psi, db);           \
+        else sweep3d_oct<R, DB_, 1, CSD, false>(t, P, gs, smem, phiE_in, phiE_out, psi, db);                \
+        return;                                                                                             \
+    }
+    if constexpr (std::is_same<Team, GridTeam>::value) {
+        if constexpr (sizeof(R) == 8 && !CSD) {
+            if (P.recip) {  // (one instantiation each: three of a group's passes)
+                if (even) sweep3d_oct<R, 10, 2, false, true>(t, P, gs, smem, phiE_in, phiE_out, psi, db);
+                else sweep3d_oct<R, 10, 1, false, true>(t, P, gs, smem, phiE_in, phiE_out, psi, db);
+                return;
+            }
+        }
+        if (db <= 6) RB_OCT_RUN(6)
+        if (sizeof(R) == 4 && db <= 10) RB_OCT_RUN(10)
+    }
+    RB_OCT_RUN(OctDB<R>::value)
+#undef RB_OCT_RUN
+}
+
+// q / s given r = 1 / s correctly rounded: Markstein's correction of q·r, the correctly rounded
+// quotient. The reciprocal does not wait for the cell's faces, the two products do.
+__device__ __forceinline__ double div_by(double q, double s, double r) {
+    const double v = q * r;
+    return fma(fma(-s, v, q), r, v);
+}
+__device__ __forceinline__ float div_by(float q, float s, float r) {
+    const float v = q * r;
+    return fmaf(fmaf(-s, v, q), r, v);
+}
+__device__ __forceinline__ double recip(double s) { return oct_div(1.0, s); }
+__device__ __forceinline__ float recip(float s) { return __frcp_rn(s); }
+
+// 2D, one-moment cells: sweep_md's wavefront with the arithmetic in R (FP64 or FP32) over an
+// angular buffer held cells fastest.
+//
+// A warp takes 32 rows of a direction, one per lane, each a column behind the lane below; the y
+// face goes up by shuffle. Lane 31 leaves its faces in shared memory for lane 0 of the warp above,
+// which runs RB_2D_K more steps behind than it must, so that one block barrier per piece of RB_2D_K
+// steps stands between the faces' stores and their loads.
+//
+// What bounds it: with one or two directions a CTA there is about one warp per scheduler, so every
+// instruction of a step counts with its latency, nx + rows + lag times. So a piece of RB_2D_K steps
+// works out its cells' coefficients (collision term, reciprocal, face factors: independent of the
+// faces) together, in registers, and a step is left with the shuffle and the cell's few dependent
+// operations. The piece's inputs come by cp.async two pieces ahead into the warp's own tile, 8 lanes
+// to a row's run of 8 cells; the outputs leave the same way.
+#define RB_2D_K 8
+// elements of a warp's tile of one array: 32 rows of K cells, padded to an odd stride
+#define RB_2D_TILE (32 * (RB_2D_K + 1))
+// bytes of the sweep's region: two tiles per warp of ψ, energy-face flux and material, then Σt (+ the
+// CSD cell term) and the factor of the incoming energy-face flux per material, and the inverse widths
+__host__ __device__ __forceinline__ long long sweep2d_bytes(int nx, int mixed, int csd) {
+    return (long long)(RB_THREADS / 32) * 2 * RB_2D_TILE * ((mixed ? 4 : 8) + (csd ? 8 : 0) + 4) + (long long)(nx + 2 * RB_MAXMAT) * (mixed ? 4 : 8);
+}
+template <typename R, bool CSD, class Team>
+__device__ __noinline__ void sweep2d_pf(Team &t, const DevProblem &P, GroupShared &gs, void *region, const double *phiE_in,
+                                        double *phiE_out, R *psi) {
+    constexpr int K = RB_2D_K, TS = RB_2D_TILE, NW = RB_THREADS / 32;
+    static_assert(K == 8, "a piece is 8 cells of a row: 8 lanes, 4 rows per copy");
+    const int nd = P.nd, nx = P.nx, ny = P.ny, nfm = P.nfmax, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ncta = (int)t.ncta, crank = (int)t.crank;
-    // directions dealt in contiguous blocks, so the directions of a CTA are neighbours in ψ
     const int dlo = (int)((long long)nd * crank / ncta), dhi = (int)((long long)nd * (crank + 1) / ncta);
     const int my_dirs = dhi - dlo;
-    const int Rr = ny < (int)blockDim.x ? ny : (int)blockDim.x;  // rows per direction
-    int D = (int)blockDim.x / Rr;
+    if (my_dirs == 0) return;
+    const int nwd = min(NW, (ny + 31) / 32), rows = 32 * nwd;  // warps of a direction, rows of a block
+    int D = NW / nwd;                                          // directions in work
     const int dmax = RB_TILE_DOUBLES * (int)(sizeof(double) / sizeof(R)) / nx;  // y-face slots
     if (D > dmax) D = dmax;
-    const int nrb = (ny + Rr - 1) / Rr;
-    const long long sstride = md_scratch_stride(P);
+    const int nrb = (ny + rows - 1) / rows;
+    const int npiece = (nx + 31 + (nwd - 1) * (32 + K) + K - 1) / K;
+    const long long sstride = md_scratch_stride(P), sn = P.psi_sn;
     const long long xin = md_in_offset(P, 0), yin = md_in_offset(P, 1);
     R *yface = reinterpret_cast<R *>(gs.tile);  // [D][nx]
     const R w1x = (R)P.w1[0], w1y = (R)P.w1[1], w1e = (R)P.w1[3];
     const R esa = CSD ? (R)P.EsA[0] : R(0), esb = CSD ? (R)P.EsB[0] : R(0), eout = CSD ? (R)P.Eout[0] : R(0);
-    for (int k0 = 0; k0 < my_dirs; k0 += D) {
-        const int dl = threadIdx.x / Rr, r = threadIdx.x % Rr;
-        const bool active = dl < D && k0 + dl < my_dirs;
-        const int n = dlo + k0 + dl;
-        const double mu = active ? P.cosv[n] : 0.0, eta = active ? P.cosv[nd + n] : 0.0;
-        const bool fx = mu >= 0.0, fy = eta >= 0.0;
-        R gx = R(0), gy = R(0), sx = R(0), sy = R(0), ox = R(0), oy = R(0);
-        if (active) {
-            gx = (R)(fabs(mu) * P.G[(long long)n * 3]);
-            gy = (R)(fabs(eta) * P.G[(long long)n * 3 + 1]);
-            sx = (R)(fabs(mu) * P.Gsrc[((long long)n * 3) * nfm]);
-            sy = (R)(fabs(eta) * P.Gsrc[((long long)n * 3 + 1) * nfm]);
-            ox = (R)P.Gout[((long long)n * 3) * nfm];
-            oy = (R)P.Gout[((long long)n * 3 + 1) * nfm];
+    const int *mat = P.mat;
+    const double *dxp = P.dx;
+    // this warp's tiles [2][TS], and the inverse widths
+    double *es = reinterpret_cast<double *>(region) + warp * 2 * TS;
+    R *qs0 = reinterpret_cast<R *>(reinterpret_cast<double *>(region) + (CSD ? NW * 2 * TS : 0)), *qs = qs0 + warp * 2 * TS;
+    int *ms0 = reinterpret_cast<int *>(qs0 + NW * 2 * TS), *ms = ms0 + warp * 2 * TS;
+    R *mS = reinterpret_cast<R *>(ms0 + NW * 2 * TS), *mQ = mS + RB_MAXMAT, *idxs = mQ + RB_MAXMAT;
+    __syncthreads();
+    for (int m = tid; m < P.nmat; m += blockDim.x) {
+        R S = (R)gs.sigt[m], sq = R(0);
+        if (CSD) {
+            S = (R)P.scsd[m] + S;
+            sq = esa * (R)gs.sp[m] - esb * (R)gs.sm[m];
         }
-        double *scr = P.fexit + (active ? (long long)n * sstride : 0);
+        mS[m] = S;
+        mQ[m] = sq;
+    }
+    for (int i = tid; i < nx; i += blockDim.x) idxs[i] = (R)(1.0 / dxp[i]);
+    const int dl = warp / nwd, jw = warp % nwd;  // this warp's direction and its place among its warps
+    const int lag0 = jw * (32 + K);              // steps the warp's first row runs behind
+    for (int k0 = 0; k0 < my_dirs; k0 += D) {
+        const bool active = dl < D && k0 + dl < my_dirs;
+        const int n = dlo + k0 + (active ? dl : 0);
+        const double mu = P.cosv[n], eta = P.cosv[nd + n];
+        const bool fx = mu >= 0.0, fy = eta >= 0.0;
+        const R gx = (R)(fabs(mu) * P.G[(long long)n * 3]), gy = (R)(fabs(eta) * P.G[(long long)n * 3 + 1]);
+        const R sx = (R)(fabs(mu) * P.Gsrc[((long long)n * 3) * nfm]), sy = (R)(fabs(eta) * P.Gsrc[((long long)n * 3 + 1) * nfm]);
+        const R ox = (R)P.Gout[((long long)n * 3) * nfm], oy = (R)P.Gout[((long long)n * 3 + 1) * nfm];
+        double *scr = P.fexit + (long long)n * sstride;
         double *exx = scr, *exy = exx + (long long)ny * nfm;
-        R *yf = yface + (long long)dl * nx;
+        R *yf = yface + (long long)(active ? dl : 0) * nx;
+        R *pn = psi + n * sn;
+        const double *ein = (CSD && phiE_in) ? phiE_in + n * sn : nullptr;
+        double *eou = (CSD && phiE_out) ? phiE_out + n * sn : nullptr;
+        __syncthreads();  // the previous round's readers of the face slots are done
+        if (active)       // the first row's Y faces: the incoming fluxes of boundary_in_phase
+            for (int i = 32 * jw + lane; i < nx; i += rows) yf[i] = (R)scr[yin + (long long)(fx ? i : nx - 1 - i) * nfm];
         for (int rb = 0; rb < nrb; rb++) {
-            const int iyy = rb * Rr + r;
+            const int iy0 = rb * rows + 32 * jw, iyy = iy0 + lane;  // the warp's first row, this row
             const bool row = active && iyy < ny;
             const int iy = fy ? iyy : ny - 1 - iyy;
             const R idy = row ? (R)(1.0 / P.dy[iy]) : R(0);
-            R F0 = R(0), qp = R(0), fep = R(0), idxp = R(0);
-            int mp = 0;
-            if (row) {  // the inputs of the row's first cell; the later ones are loaded a step ahead
-                const int ix0 = fx ? 0 : nx - 1;
-                const long long c0 = ix0 + (long long)nx * iy;
-                qp = (R)psi[n + (long long)nd * c0];
-                if (CSD) fep = phiE_in ? (R)phiE_in[n + (long long)nd * c0] : R(0);
-                mp = P.mat[c0];
-                idxp = (R)(1.0 / P.dx[ix0]);
-            }
-            for (int s = 0; s < nx + Rr - 1; s++) {
-                const int ixx = s - r;
-                R qn = R(0), fen = R(0), idxn = R(0);
-                int mn_ = 0;
-                const bool nxt = row && ixx >= 0 && ixx + 1 < nx;
-                if (nxt) {
-                    const int ixn = fx ? ixx + 1 : nx - 2 - ixx;
-                    const long long cn = ixn + (long long)nx * iy;
-                    qn = (R)psi[n + (long long)nd * cn];
-                    if (CSD) fen = phiE_in ? (R)phiE_in[n + (long long)nd * cn] : R(0);
-                    mn_ = P.mat[cn];
-                    idxn = (R)(1.0 / P.dx[ixn]);
-                }
-                if (row && ixx >= 0 && ixx < nx) {
-                    const int ix = fx ? ixx : nx - 1 - ixx;
-                    const long long c = ix + (long long)nx * iy;
-                    // X face of the row and Y face of the column (sn_sweep_2D.jl:71-132): the
-                    // incoming fluxes of boundary_in_phase
-                    if (ixx == 0) F0 = (R)scr[xin + (long long)iy * nfm];
-                    const R F1 = iyy == 0 ? (R)scr[yin + (long long)ix * nfm] : yf[ixx];
-                    const int m = mp;
-                    R S = (R)gs.sigt[m], srcE = R(0);
-                    if (CSD) {
-                        S = (R)P.scsd[m] + S;
-                        srcE = esa * (R)gs.sp[m] - esb * (R)gs.sm[m];
+            const bool last = iyy == ny - 1, keep = lane == 31 || last;  // rows whose faces go on
+            // Element i of this lane in a piece: row 4·i + lane/8, step lane%8. Its column in sweep
+            // order is (first step of the piece) + eb − 4·i, its cell e0 + i·de + (first step)·dx1.
+            const int er = lane >> 3, ec = lane & 7;
+            const int eb = ec - lag0 - er, rmax = active ? ny - iy0 - er : 0;  // rows: 4·i < rmax
+            const int dx1 = fx ? 1 : -1;
+            const long long e0 = (long long)nx * (fy ? iy0 + er : ny - 1 - iy0 - er) + (fx ? eb : nx - 1 - eb);
+            const long long de = 4LL * (fy ? nx : -nx) - 4LL * dx1;
+            const int eo = er * (K + 1) + ec;
+            auto load = [&](int p) {  // the inputs of piece p
+                const int b = (p & 1) * TS + eo, c0 = p * K + eb;
+                const long long g = e0 + (long long)(p * K) * dx1;
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (4 * i < rmax && (unsigned)(c0 - 4 * i) < (unsigned)nx) {
+                        const long long c = g + i * de;
+                        cp_async<sizeof(R)>(qs + b + i * 4 * (K + 1), pn + c);
+                        if (CSD && ein) cp_async<8>(es + b + i * 4 * (K + 1), ein + c);
+                        cp_async<4>(ms + b + i * 4 * (K + 1), mat + c);
                     }
-                    const R idx = idxp;
-                    S = S + gx * idx + gy * idy;
-                    R q = qp + (sx * idx) * F0 + (sy * idy) * F1;
-                    if (CSD) q -= srcE * fep;
-                    const R v = q / S;
-                    F0 = w1x * F0 + ox * v;
-                    const R F1o = w1y * F1 + oy * v;
-                    psi[n + (long long)nd * c] = (PS)v;
-                    if (CSD) phiE_out[n + (long long)nd * c] = (double)(w1e * fep + eout * v);
-                    yf[ixx] = F1o;
-                    if (ixx == nx - 1) exx[(long long)iy * nfm] = (double)F0;
-                    if (iyy == ny - 1) exy[(long long)ix * nfm] = (double)F1o;
+                cp_async_commit();
+            };
+            auto store = [&](int p) {  // the outputs of piece p
+                const int b = (p & 1) * TS + eo, c0 = p * K + eb;
+                const long long g = e0 + (long long)(p * K) * dx1;
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (4 * i < rmax && (unsigned)(c0 - 4 * i) < (unsigned)nx) {
+                        const long long c = g + i * de;
+                        pn[c] = qs[b + i * 4 * (K + 1)];
+                        if (CSD && eou) eou[c] = es[b + i * 4 * (K + 1)];
+                    }
+            };
+            load(0);
+            load(1);
+            R F0 = row ? (R)scr[xin + (long long)iy * nfm] : R(0), Fy = R(0);
+            const R cay = sy * idy;
+            for (int p = 0; p < npiece; p++) {
+                cp_async_wait<1>();
+                __syncthreads();  // the piece in every lane's view; the faces that lane 0 takes are stored
+                const int c0 = p * K - lag0 - lane;  // this row's column at the piece's first step
+                R *q = qs + (p & 1) * TS + lane * (K + 1);
+                double *e = es + (p & 1) * TS + lane * (K + 1);
+                const int *mm = ms + (p & 1) * TS + lane * (K + 1);
+                R cS[K], cr[K], cq[K], cax[K], cf[K], ce[CSD ? K : 1], cQ[CSD ? K : 1];
+                bool in[K];
+#pragma unroll
+                for (int u = 0; u < K; u++) {
+                    in[u] = row && (unsigned)(c0 + u) < (unsigned)nx;
+                    const int x = in[u] ? c0 + u : 0, m = in[u] ? mm[u] : 0;
+                    const R ix = idxs[fx ? x : nx - 1 - x];
+                    R S = mS[m];
+                    S = S + gx * ix + gy * idy;
+                    cS[u] = S;
+                    cq[u] = q[u];
+                    cax[u] = sx * ix;
+                    cf[u] = lane == 0 ? yf[x] : R(0);
+                    if (CSD) {
+                        ce[CSD ? u : 0] = ein ? (R)e[u] : R(0);
+                        cQ[CSD ? u : 0] = mQ[m];
+                    }
                 }
-                if (nxt) { qp = qn; fep = fen; mp = mn_; idxp = idxn; }
-                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < K; u++) cr[u] = recip(cS[u]);
+#pragma unroll
+                for (int u = 0; u < K; u++) {
+                    // X face of the row and Y face of the column (sn_sweep_2D.jl:71-132)
+                    const R up = __shfl_up_sync(0xffffffffu, Fy, 1);
+                    const R F1 = lane == 0 ? cf[u] : up;
+                    R qq = cq[u] + cax[u] * F0 + cay * F1;
+                    if (CSD) qq -= cQ[CSD ? u : 0] * ce[CSD ? u : 0];
+                    const R v = div_by(qq, cS[u], cr[u]);
+                    const R F0o = w1x * F0 + ox * v;
+                    Fy = w1y * F1 + oy * v;
+                    F0 = in[u] ? F0o : F0;
+                    q[u] = v;
+                    if (CSD && eou) e[u] = (double)(w1e * ce[CSD ? u : 0] + eout * v);
+                    if (keep && in[u]) yf[c0 + u] = Fy;
+                }
+                __syncwarp();
+                store(p);
+                __syncwarp();  // the tile takes the piece after the next
+                load(p + 2);
             }
+            if (row) exx[(long long)iy * nfm] = (double)F0;
+            cp_async_wait<0>();
+            __syncthreads();
+            if (active && rb == nrb - 1)  // the last row's faces leave the domain
+                for (int i = 32 * jw + lane; i < nx; i += rows) exy[(long long)(fx ? i : nx - 1 - i) * nfm] = (double)yf[i];
         }
     }
+}
+
+// 2D cells of NM moments (FP64): the same wavefront. The cell matrix S = Σt·I + Σ_a h_a·G_a + Scsd
+// of flux_2D_BTE / flux_2D_BFP (sn_2D_bte.jl:35-116, sn_2D_bfp.jl:45-154) depends on the direction,
+// the material and the widths only, so a lane keeps its inverse in registers along the row and
+// factors again where the material or a width changes; a cell is then a product with the inverse.
+// (The run-time shaped solve, which stays for the other shapes, eliminates every cell's matrix in
+// local memory: 9.4 us a step at 41×30, S6, four moments.)
+#define RB_2DHI_PF 4
+template <int NM, int NF, int NE, bool CSD>
+struct Sweep2dHi {
+    // doubles of the direction tables: G, Gsrc, Gout of both axes, the energy-face factors
+    static constexpr int TAB = 2 * (NM * NM + 2 * NM * NF) + (CSD ? 3 * NM * NE : 0);
+    static constexpr int SLOT = NM + (CSD ? NE : 0);
+    static constexpr long long bytes = 8LL * (8 * TAB + (long long)RB_2DHI_PF * SLOT * RB_THREADS) + 4LL * RB_2DHI_PF * RB_THREADS;
+    // a thread's slot is NM consecutive values, copied and stored in pairs where NM is even
+    static constexpr int V = NM % 2 == 0 ? 2 : 1, VE = NE % 2 == 0 ? 2 : 1;
+};
+template <int NM, int NF, int NE, bool CSD, class Team>
+__device__ __noinline__ void sweep2d_hi(Team &t, const DevProblem &P, GroupShared &gs, void *region, const double *phiE_in,
+                                        double *phiE_out) {
+    using L = Sweep2dHi<NM, NF, NE, CSD>;
+    constexpr int PF = RB_2DHI_PF, K = RB_2D_K, GG = NM * NM, GF = NM * NF;
+    const int nd = P.nd, nx = P.nx, ny = P.ny, nfm = P.nfmax, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ncta = (int)t.ncta, crank = (int)t.crank;
+    const int dlo = (int)((long long)nd * crank / ncta), dhi = (int)((long long)nd * (crank + 1) / ncta);
+    const int my_dirs = dhi - dlo;
+    if (my_dirs == 0) return;
+    const int nwarp = RB_THREADS / 32;
+    const int nwd = min(nwarp, (ny + 31) / 32), rows = 32 * nwd;
+    int D = nwarp / nwd;
+    const int dmax = RB_TILE_DOUBLES / (nx * NF);  // y-face slots (at least one: checked at upload)
+    if (D > dmax) D = dmax;
+    const int nrb = (ny + rows - 1) / rows;
+    const int nsteps = nx + 31 + (nwd - 1) * (32 + K);
+    const long long sstride = md_scratch_stride(P);
+    const long long xin = md_in_offset(P, 0), yin = md_in_offset(P, 1);
+    double *yface = gs.tile;  // [D][nx][NF]
+    double *tabs = reinterpret_cast<double *>(region);
+    double *qs = tabs + 8 * L::TAB + tid * L::V;        // [PF][NM / V][threads][V]
+    double *es = tabs + 8 * L::TAB + PF * NM * RB_THREADS + tid * L::VE;  // [PF][NE / VE][threads][VE]
+    int *ms = reinterpret_cast<int *>(tabs + 8 * L::TAB + PF * L::SLOT * RB_THREADS) + tid;  // [PF][threads]
+    double *dxs = reinterpret_cast<double *>(ms - tid + PF * RB_THREADS);  // [nx] widths
+    auto qat = [](int o, int j) { return ((o * (NM / L::V) + j / L::V) * RB_THREADS) * L::V + j % L::V; };
+    auto eat = [](int o, int e) { return ((o * (NE / L::VE) + e / L::VE) * RB_THREADS) * L::VE + e % L::VE; };
+    for (int i = tid; i < nx; i += blockDim.x) dxs[i] = P.dx[i];
+    const double w1x = P.w1[0], w1y = P.w1[1], w1e = P.w1[3];
+    const int *mat = P.mat;
+    const int dl = warp / nwd, jw = warp % nwd;
+    const int lag = jw * (32 + K) + lane;
+    for (int k0 = 0; k0 < my_dirs; k0 += D) {
+        const bool active = dl < D && k0 + dl < my_dirs;
+        const int n = dlo + k0 + (active ? dl : 0);
+        const double amu = fabs(P.cosv[n]), aeta = fabs(P.cosv[nd + n]);
+        const bool fx = P.cosv[n] >= 0.0, fy = P.cosv[nd + n] >= 0.0;
+        double *scr = P.fexit + (long long)n * sstride;
+        double *exx = scr, *exy = exx + (long long)ny * nfm;
+        double *yf = yface + (long long)(active ? dl : 0) * nx * NF;
+        double *T = tabs + (active ? dl : 0) * L::TAB;  // [a]: G, Gsrc (j + NM·f), Gout (f + NF·j); then EsA, EsB, Eout
+        __syncthreads();  // the previous round's readers are done
+        if (active) {
+            for (int e = 32 * jw + lane; e < L::TAB; e += rows) {
+                constexpr int AX = GG + 2 * GF;
+                double v;
+                if (e < 2 * AX) {
+                    const int a = e / AX, o = e % AX;
+                    const long long blk = (long long)n * 3 + a;
+                    v = o < GG ? P.G[blk * GG + o] : (o < GG + GF ? P.Gsrc[blk * NM * nfm + o - GG] : P.Gout[blk * NM * nfm + o - GG - GF]);
+                } else {
+                    const int o = e - 2 * AX;
+                    v = o < NM * NE ? P.EsA[o] : (o < 2 * NM * NE ? P.EsB[o - NM * NE] : P.Eout[o - 2 * NM * NE]);
+                }
+                T[e] = v;
+            }
+            for (int i = 32 * jw + lane; i < nx; i += rows)
+                for (int f = 0; f < NF; f++) yf[i * NF + f] = scr[yin + (long long)(fx ? i : nx - 1 - i) * nfm + f];
+        }
+        __syncthreads();
+        const double *Tx = T, *Ty = T + GG + 2 * GF, *TE = T + 2 * (GG + 2 * GF);
+        for (int rb = 0; rb < nrb; rb++) {
+            const int iyy = rb * rows + 32 * jw + lane;
+            const bool row = active && iyy < ny;
+            const int iy = fy ? iyy : ny - 1 - iyy;
+            const double hy = row ? aeta / P.dy[iy] : 0.0;
+            const long long c0 = row ? (long long)nx * iy : 0;
+            double *prow = P.psi + n * P.psi_sn + NM * c0;
+            const double *ein = (CSD && phiE_in) ? phiE_in + n * P.pe_sn + NE * c0 : nullptr;
+            double *eou = (CSD && phiE_out) ? phiE_out + n * P.pe_sn + NE * c0 : nullptr;
+            const bool last = iyy == ny - 1, top = lane == 31 && !last;
+            auto load = [&](int s) {
+                const int ixx = s - lag, o = s % PF;
+                if (row && ixx >= 0 && ixx < nx) {
+                    const int ix = fx ? ixx : nx - 1 - ixx;
+#pragma unroll
+                    for (int j = 0; j < NM; j += L::V) cp_async<8 * L::V>(qs + qat(o, j), prow + ix * NM + j);
+                    if (CSD && ein)
+#pragma unroll
+                        for (int e = 0; e < NE; e += L::VE) cp_async<8 * L::VE>(es + eat(o, e), ein + ix * NE + e);
+                    cp_async<4>(ms + o * RB_THREADS, mat + c0 + ix);
+                }
+                cp_async_commit();
+            };
+            // the direction's face factors stay in registers along the row
+            double gsx[GF], gsy[GF], gox[GF], goy[GF];
+#pragma unroll
+            for (int e = 0; e < GF; e++) {
+                gsx[e] = Tx[GG + e];
+                gsy[e] = hy * Ty[GG + e];
+                gox[e] = Tx[GG + GF + e];
+                goy[e] = Ty[GG + GF + e];
+            }
+            double Si[NM * NM], F0[NF], Fy[NF], hk = -1.0, hx = 0.0, esa[CSD ? NM * NE : 1];
+            int mk = -1;
+#pragma unroll
+            for (int e = 0; e < NM * NM; e++) Si[e] = 0.0;
+#pragma unroll
+            for (int f = 0; f < NF; f++) {
+                F0[f] = row ? scr[xin + (long long)iy * nfm + f] : 0.0;
+                Fy[f] = 0.0;
+            }
+            for (int s = 0; s < PF; s++) load(s);
+            for (int s = 0; s < nsteps; s++) {
+                const int ixx = s - lag, o = s % PF;
+                const bool in = row && ixx >= 0 && ixx < nx;
+                if (s % K == 0) __syncthreads();  // the faces that lane 0 loads in these steps are stored
+                cp_async_wait<PF - 1>();
+                double F1[NF];
+#pragma unroll
+                for (int f = 0; f < NF; f++) F1[f] = __shfl_up_sync(0xffffffffu, Fy[f], 1);
+                if (in) {
+                    const int ix = fx ? ixx : nx - 1 - ixx;
+                    const int m = ms[o * RB_THREADS];
+                    const double dxc = dxs[ix];
+                    if (m != mk || dxc != hk) {  // another kind of cell: its inverse
+                        mk = m;
+                        hk = dxc;
+                        hx = amu / dxc;
+                        double S[NM * NM], q[NM][NM];
+#pragma unroll
+                        for (int i = 0; i < NM; i++)
+#pragma unroll
+                            for (int j = 0; j < NM; j++) {
+                                S[i + NM * j] = (CSD ? P.scsd[(long long)m * GG + i + NM * j] : 0.0) + (i == j ? gs.sigt[m] : 0.0) +
+                                                hx * Tx[i + NM * j] + hy * Ty[i + NM * j];
+                                q[i][j] = i == j ? 1.0 : 0.0;
+                            }
+                        lu_solve<double, NM, NM>(S, q);
+#pragma unroll
+                        for (int j = 0; j < NM; j++)
+#pragma unroll
+                            for (int i = 0; i < NM; i++) Si[i + NM * j] = q[j][i];
+                        if (CSD)
+#pragma unroll
+                            for (int e = 0; e < NM * NE; e++) esa[CSD ? e : 0] = TE[e] * gs.sp[m] - TE[NM * NE + e] * gs.sm[m];
+                    }
+                    if (lane == 0)
+#pragma unroll
+                        for (int f = 0; f < NF; f++) F1[f] = yf[ixx * NF + f];
+                    double q[NM], v[NM], fe[CSD ? NE : 1];
+#pragma unroll
+                    for (int j = 0; j < NM; j++) {
+                        double ax = 0.0, ay = 0.0;
+#pragma unroll
+                        for (int f = 0; f < NF; f++) {
+                            ax += gsx[j + NM * f] * F0[f];
+                            ay += gsy[j + NM * f] * F1[f];
+                        }
+                        q[j] = qs[qat(o, j)] + hx * ax + ay;
+                    }
+                    if constexpr (CSD) {
+#pragma unroll
+                        for (int e = 0; e < NE; e++) fe[e] = ein ? es[eat(o, e)] : 0.0;
+#pragma unroll
+                        for (int j = 0; j < NM; j++)
+#pragma unroll
+                            for (int e = 0; e < NE; e++) q[j] -= esa[j + NM * e] * fe[e];
+                    }
+#pragma unroll
+                    for (int i = 0; i < NM; i++) {
+                        double x = 0.0;
+#pragma unroll
+                        for (int j = 0; j < NM; j++) x += Si[i + NM * j] * q[j];
+                        v[i] = x;
+                    }
+#pragma unroll
+                    for (int f = 0; f < NF; f++) {
+                        double x = w1x * F0[f], y = w1y * F1[f];
+#pragma unroll
+                        for (int j = 0; j < NM; j++) {
+                            x += gox[f + NF * j] * v[j];
+                            y += goy[f + NF * j] * v[j];
+                        }
+                        F0[f] = x;
+                        Fy[f] = y;
+                    }
+#pragma unroll
+                    for (int j = 0; j < NM; j += L::V) {
+                        if (L::V == 2) *reinterpret_cast<double2 *>(prow + ix * NM + j) = make_double2(v[j], v[j + L::V - 1]);
+                        else prow[ix * NM + j] = v[j];
+                    }
+                    if constexpr (CSD) {
+                        if (eou)
+#pragma unroll
+                            for (int e = 0; e < NE; e++) {
+                                double x = w1e * fe[e];
+#pragma unroll
+                                for (int j = 0; j < NM; j++) x += TE[2 * NM * NE + e + NE * j] * v[j];
+                                eou[ix * NE + e] = x;
+                            }
+                    }
+#pragma unroll
+                    for (int f = 0; f < NF; f++) {
+                        if (top) yf[ixx * NF + f] = Fy[f];
+                        if (ixx == nx - 1) exx[(long long)iy * nfm + f] = F0[f];
+                        if (last) exy[(long long)ix * nfm + f] = Fy[f];
+                    }
+                }
+                __syncwarp();
+                load(s + PF);
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+        }
+    }
+}
+
+// 2D cells of several moments: the compiled shapes (linear closures: full coupling, without and with
+// an energy closure of order 1, and without cross terms), false where the shape is another one.
+// sweep2d_hi_bytes is the region they need.
+__host__ __device__ __forceinline__ int sweep2d_hi_shape(const DevProblem &P) {
+    if (P.ndims != 2 || P.nmf[0] != P.nmf[1] || P.nfmax != P.nmf[0]) return 0;
+    if (!P.csd && P.nm5 == 4 && P.nmf[0] == 2) return 1;
+    if (!P.csd && P.nm5 == 3 && P.nmf[0] == 2) return 2;
+    if (P.csd && P.nm5 == 4 && P.nmf[0] == 2 && P.nm4 == 4) return 3;
+    return 0;
+}
+__host__ __device__ __forceinline__ long long sweep2d_hi_bytes(const DevProblem &P) {
+    const int k = sweep2d_hi_shape(P);
+    const long long fixed = k == 1 ? Sweep2dHi<4, 2, 1, false>::bytes
+                                   : (k == 2 ? Sweep2dHi<3, 2, 1, false>::bytes : Sweep2dHi<4, 2, 4, true>::bytes);
+    return k == 0 ? 0 : fixed + 8LL * P.nx;
+}
+template <class Team>
+__device__ __forceinline__ bool sweep2d_hi_run(Team &t, const DevProblem &P, GroupShared &gs, void *region, long long bytes,
+                                               const double *pE, double *phiE_out) {
+    const int k = sweep2d_hi_shape(P);
+    if (k == 0 || bytes < sweep2d_hi_bytes(P)) return false;
+    if (k == 1) sweep2d_hi<4, 2, 1, false>(t, P, gs, region, pE, phiE_out);
+    else if (k == 2) sweep2d_hi<3, 2, 1, false>(t, P, gs, region, pE, phiE_out);
+    else sweep2d_hi<4, 2, 4, true>(t, P, gs, region, pE, phiE_out);
+    return true;
 }
 
 // The pass for 2D and 3D problems. mixed: FP32 angular buffer, products and sweep where the
@@ -562,41 +1024,47 @@ __device__ __noinline__ void pass_md(Team &t, const DevProblem &P, GroupShared &
                         double *phiE_out, int mixed) {
     const bool one = one_moment_md(P);
     const bool oct = oct3d_ok(P, (int)t.ncta, smem_bytes, mixed);
-    const int mx = (mixed && one && (P.ndims == 2 || oct)) ? 1 : 0;
+    const bool pf = P.ndims == 2 && one && smem_bytes >= sweep2d_bytes(P.nx, 0, P.csd);
+    const int mx = (mixed && (pf || oct)) ? 1 : 0;
     // the mixed form's products go to the tensor cores where the CTA holds TMEM and they fit
     if (!mx || !m2d_tc(t, P, gs, gs.tc, smem, smem_bytes, zin, homog ? nullptr : P.qnout))
-        m2d_tiles(t, P, gs, zin, homog ? nullptr : P.qnout, 1, mx);
+        m2d_tiles(t, P, gs, smem, smem_bytes, zin, homog ? nullptr : P.qnout, P.psi, 1, mx);
     const int np_source = homog ? 0 : P.np_source;
     const double *pE = (P.csd && !homog) ? phiE_in : nullptr;
-    const bool newsweep = (P.ndims == 3 && oct) || (P.ndims == 2 && one);
-    if (newsweep) boundary_in_phase(t, P, zin, np_source, ig);
+    const bool hi = sweep2d_hi_shape(P) != 0 && smem_bytes >= sweep2d_hi_bytes(P);
+    const bool newsweep = (P.ndims == 3 && oct) || (P.ndims == 2 && (pf || hi));
+    // the faces' products stage in the region, or in GroupShared where there is none
+    const bool own = smem_bytes >= (long long)sizeof(gs.tile);
+    void *fr = own ? smem : (void *)gs.tile;
+    const long long frb = own ? smem_bytes : (long long)sizeof(gs.tile);
+    if (newsweep) boundary_in_phase(t, P, fr, frb, zin, np_source, ig);
     t.sync();
     if (P.ndims == 3 && oct) {
         if (mx) {
-            if (P.csd) sweep3d_oct<float, float, true>(t, P, gs, smem, zin, np_source, pE, phiE_out, ig, P.psi32);
-            else sweep3d_oct<float, float, false>(t, P, gs, smem, zin, np_source, pE, phiE_out, ig, P.psi32);
+            if (P.csd) sweep3d_run<float, true>(t, P, gs, smem, pE, phiE_out, P.psi32);
+            else sweep3d_run<float, false>(t, P, gs, smem, pE, phiE_out, P.psi32);
         } else {
-            if (P.csd) sweep3d_oct<double, double, true>(t, P, gs, smem, zin, np_source, pE, phiE_out, ig, P.psi);
-            else sweep3d_oct<double, double, false>(t, P, gs, smem, zin, np_source, pE, phiE_out, ig, P.psi);
+            if (P.csd) sweep3d_run<double, true>(t, P, gs, smem, pE, phiE_out, P.psi);
+            else sweep3d_run<double, false>(t, P, gs, smem, pE, phiE_out, P.psi);
         }
-    } else if (P.ndims == 2 && one) {
+    } else if (pf) {
         if (mx) {
-            if (P.csd) sweep2d_pf<float, float, true>(t, P, gs, zin, np_source, pE, phiE_out, ig, P.psi32);
-            else sweep2d_pf<float, float, false>(t, P, gs, zin, np_source, pE, phiE_out, ig, P.psi32);
+            if (P.csd) sweep2d_pf<float, true>(t, P, gs, smem, pE, phiE_out, P.psi32);
+            else sweep2d_pf<float, false>(t, P, gs, smem, pE, phiE_out, P.psi32);
         } else {
-            if (P.csd) sweep2d_pf<double, double, true>(t, P, gs, zin, np_source, pE, phiE_out, ig, P.psi);
-            else sweep2d_pf<double, double, false>(t, P, gs, zin, np_source, pE, phiE_out, ig, P.psi);
+            if (P.csd) sweep2d_pf<double, true>(t, P, gs, smem, pE, phiE_out, P.psi);
+            else sweep2d_pf<double, false>(t, P, gs, smem, pE, phiE_out, P.psi);
         }
     } else if (P.ndims == 3) {
         if (one && !P.csd) sweep_3d_tiles<CellMDfix<1, 1, 1, false, 3>, 1, 1, 1>(t, P, gs, zin, np_source, pE, phiE_out, ig);
         else if (one) sweep_3d_tiles<CellMDfix<1, 1, 1, true, 3>, 1, 1, 1>(t, P, gs, zin, np_source, pE, phiE_out, ig);
         else sweep_3d_tiles<CellMDgen, RB_MAXNM, RB_MAXFACE, RB_MAXFACE>(t, P, gs, zin, np_source, pE, phiE_out, ig);
-    } else {
+    } else if (!hi || !sweep2d_hi_run(t, P, gs, smem, smem_bytes, pE, phiE_out)) {
         sweep_md<CellMDgen, RB_MAXNM, RB_MAXFACE, RB_MAXFACE>(t, P, gs, zin, np_source, pE, phiE_out, ig);
     }
     t.sync();
-    if (!mx || !d2m_tc(t, P, gs.tc, smem, smem_bytes, zin, zout, matvec)) d2m_tiles(t, P, gs, zin, zout, matvec, mx);
-    boundary_out_md(t, P, zin, zout, matvec);
+    if (!mx || !d2m_tc(t, P, gs.tc, smem, smem_bytes, zin, zout, matvec)) d2m_tiles(t, P, gs, smem, smem_bytes, zin, zout, matvec, mx);
+    boundary_out_md(t, P, fr, frb, zin, zout, matvec);
     t.sync();
 }
 

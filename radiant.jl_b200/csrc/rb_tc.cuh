@@ -145,9 +145,9 @@ __host__ __device__ constexpr int round16(int n) { return (n + 15) & ~15; }
 }  // namespace tc
 
 // One 16-K half chunk of a column into registers: k0 = first K (stacked over the parts: part
-// k / nkp, index k % nkp), X[col·ldx + index], times scale(part, col, index); zero past K.
+// k / nkp, index k % nkp), X[col·ldx + index·sx], times scale(part, col, index); zero past K.
 template <class TX, class Scale>
-__device__ __forceinline__ void tc_load_half(float (&xv)[16], const TX *X, long long ldx, long long col, bool colok,
+__device__ __forceinline__ void tc_load_half(float (&xv)[16], const TX *X, long long sx, long long ldx, long long col, bool colok,
                                              int k0, int nk, int nkp, bool vec, Scale scale) {
     const int part = k0 / nkp, kk0 = k0 % nkp;
     if (colok && vec && (kk0 * (int)sizeof(TX)) % 16 == 0 && kk0 + 16 <= nkp && k0 + 16 <= nk) {
@@ -178,7 +178,7 @@ __device__ __forceinline__ void tc_load_half(float (&xv)[16], const TX *X, long 
         float x = 0.0f;
         if (colok && k < nk) {
             const int p = k / nkp, kk = k % nkp;
-            x = (float)(scale(p, col, kk) * (double)X[col * ldx + kk]);
+            x = (float)(scale(p, col, kk) * (double)X[col * ldx + kk * sx]);
         }
         xv[e] = x;
     }
@@ -191,7 +191,7 @@ __device__ __forceinline__ void tc_load_half(float (&xv)[16], const TX *X, long 
 // does not fit.
 template <class TX, class Team, class Scale, class Epi>
 __device__ bool tc_product(Team &t, TcState &ts, unsigned char *sm, long long sm_bytes, const float *opA, int nj,
-                           int nkp, int parts, const TX *X, long long ldx, long long ncol, Scale scale, Epi epi,
+                           int nkp, int parts, const TX *X, long long sx, long long ldx, long long ncol, Scale scale, Epi epi,
                            int *status) {
     const int NJ = tc::round16(nj), nk = nkp * parts, kch = (nk + RB_TC_KC - 1) / RB_TC_KC;
     if (!ts.ready || NJ > 256 || NJ > RB_TC_TMEM_COLS) return false;
@@ -203,7 +203,7 @@ __device__ bool tc_product(Team &t, TcState &ts, unsigned char *sm, long long sm
     float *sCol = sOp + (resident ? kch * opc : 2 * opc);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int half = tid >> 7, cm = tid & 127;  // this thread's half chunk and column of a tile
-    const bool vec = ((ldx * (long long)sizeof(TX)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
+    const bool vec = sx == 1 && ((ldx * (long long)sizeof(TX)) % 16 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
     const uint32_t IDESC = tc::idesc_tf32(RB_TC_M, NJ);
     if (resident) {  // the whole operator, once
         const float4 *src = reinterpret_cast<const float4 *>(opA);
@@ -221,7 +221,7 @@ __device__ bool tc_product(Team &t, TcState &ts, unsigned char *sm, long long sm
         for (int kc = 0; kc < kch; kc++, g++) {
             const int s = g & 1;
             float xv[16];
-            tc_load_half(xv, X, ldx, col, colok, kc * RB_TC_KC + 16 * half, nk, nkp, vec, scale);
+            tc_load_half(xv, X, sx, ldx, col, colok, kc * RB_TC_KC + 16 * half, nk, nkp, vec, scale);
             // the stage's previous MMAs are done
             if (pend & (1 << s)) {
                 if (!tc::mbar_wait(&ts.mbar[s], (ph >> s) & 1) && tid == 0) atomicOr(status, RB_DEV_TIMEOUT);
@@ -317,7 +317,17 @@ __device__ bool m2d_tc(Team &t, const DevProblem &P, GroupShared &gs, TcState &t
         return part == 0 ? ys[(long long)m * np + k] : tg[m];
     };
     const bool v4 = (nd % 4) == 0, v2 = (nd % 2) == 0;
+    const long long sn = P.psi_sn;
     auto epi = [=] __device__(long long col, int j0, const float (&a)[8]) {
+        if (sn != 1) {  // cells fastest: neighbouring lanes hold neighbouring columns
+            double pv[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) pv[q] = (add && j0 + q < nd) ? add[col + (j0 + q) * sn] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (j0 + q < nd) psi[col + (j0 + q) * sn] = (float)(pv[q] + (double)a[q]);
+            return;
+        }
         float *dst = psi + col * nd + j0;
         const double *pre = add ? add + col * nd + j0 : nullptr;
         float o[8];
@@ -342,7 +352,7 @@ __device__ bool m2d_tc(Team &t, const DevProblem &P, GroupShared &gs, TcState &t
         }
     };
     return tc_product(t, ts, reinterpret_cast<unsigned char *>(smem), smem_bytes, P.tc_m2d, nd, np, parts, zin,
-                      (long long)np, ncol, sc, epi, P.status);
+                      1, (long long)np, ncol, sc, epi, P.status);
 }
 
 // The D2M product of a mixed-form 2D/3D pass on the tensor cores (FP32 angular buffer in, FP64
@@ -377,7 +387,7 @@ __device__ bool d2m_tc(Team &t, const DevProblem &P, TcState &ts, void *smem, lo
         }
     };
     return tc_product(t, ts, reinterpret_cast<unsigned char *>(smem), smem_bytes, P.tc_d2m, np, nd, 1, P.psi32,
-                      (long long)nd, ncol, one, epi, P.status);
+                      P.psi_sn, P.psi_sc, ncol, one, epi, P.status);
 }
 
 }  // namespace rb
