@@ -26,7 +26,7 @@
 #define RB_THREADS 256
 #define RB_SCAN_NF 2      // scan path for face-moment counts up to this (every fixed 1D shape)
 #define RB_MAXCLUSTER 16
-#define RB_TILE_DOUBLES 2688  // largest staging of team_product (16-deep panels, 32x128 tile, padded)
+#define RB_TILE_DOUBLES 2688  // scratch of the phases (y-face slots, small operators, FP32 panels)
 
 namespace rb {
 
@@ -626,19 +626,15 @@ __device__ void sweep1d(Team &t, const DevProblem &P, GroupShared &gs, const dou
 }
 
 // ------------------------------------------------------------------------------------------
-// moment <-> discrete products over column tiles. A column is one (is, c) pair; the moment array
-// 𝚽[p,col] and the angular array ψ[n,col] store a column contiguously, so a tile of TC columns
-// is one contiguous block, staged in shared memory with coalesced loads. The small operators
-// (Mn, Mn·ℳ, Dn) are read through the read-only cache. Tiles are dealt to the team's CTAs.
+// The FP32 products of the mixed form on the CUDA cores (1D, and 2D/3D where no CTA holds tensor
+// memory): acc[i,col] = Σ_k Op[i,k]·s(k,col)·X[k,col] with Op = [A | B] (B optional: the
+// Fokker-Planck operator under its own per-column scale), each part in an accumulator of its own,
+// added in FP64, so that a large Fokker-Planck term and the scattering term it nearly cancels are not
+// summed in single precision. Output tiles of TR rows × TC columns are dealt to the team's CTAs; each
+// thread owns a 4×4 block of a tile and the operand panels are staged in shared memory 16 values of k
+// at a time. A thread stages the same k of every panel and the same columns of a tile, so rows,
+// columns and materials are worked out once per call and per tile.
 // ------------------------------------------------------------------------------------------
-// Team-wide product over column tiles: acc[i,col] = Σ_k Op[i,k]·w(k,col)·X[k mod nk, col] with
-// Op = [A | B] (B optional, then k runs over 2·nk): a second operator applied to X under its own
-// per-column scale is one longer contraction. In FP64 one accumulator serves both parts; in
-// FP32 each part has its own and they are added in FP64, so a large Fokker-Planck term and
-// the scattering term it nearly cancels are not summed in single precision. Output tiles of
-// TR rows × TC columns are dealt to the team's CTAs; each thread owns a 4×4 block of a tile and
-// the operand panels are staged in shared memory 16 values of k at a time, converted to the
-// compute type T (double for the plain form, float for the mixed form).
 template <class TX>
 struct ProductArgs {
     const double *A, *B;   // [ni + lda·k] operators (B may be null)
@@ -648,25 +644,19 @@ struct ProductArgs {
     long long ncol;
 };
 
-template <typename T> struct Vec4;
-template <> struct Vec4<double> {
-    __device__ static void load(const double *p, double (&o)[4]) {
-        const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
-        o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-    }
-};
-template <> struct Vec4<float> {
-    __device__ static void load(const float *p, float (&o)[4]) {
-        const float4 a = *reinterpret_cast<const float4 *>(p);
-        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-    }
+// scale of X: ys[m·nk + k] for part A, tg[m] for part B, m = mat[col / nm] (ys null: 1)
+struct Scale32 {
+    const double *ys, *tg;
+    const int *mat;
+    int nm;
 };
 
-template <typename T, class TX, class Team, class Scale, class Pre, class Store>
-__device__ void team_product(Team &t, GroupShared &gs, const ProductArgs<TX> &a, Scale scale, Pre pre, Store store) {
+template <class TX, class Team, class Pre, class Store>
+__device__ void product32(const Team &t, GroupShared &gs, const ProductArgs<TX> &a, const Scale32 &sc, Pre pre, Store store) {
     constexpr int KC = 16;
     constexpr int EA = (KC * 128 + RB_THREADS - 1) / RB_THREADS;  // operator elements per thread
     constexpr int EX = (KC * 128 + RB_THREADS - 1) / RB_THREADS;  // column elements per thread
+    static_assert(RB_THREADS % KC == 0, "a thread stages one k");
     // row tiles: the operator's rows split evenly into tiles of at most 128 (a multiple of 4), so
     // an 80-row operator is one tile of 80 rows, not 64 + 16
     const int ni4 = (a.ni + 3) & ~3;
@@ -674,85 +664,84 @@ __device__ void team_product(Team &t, GroupShared &gs, const ProductArgs<TX> &a,
     const int TR = ((ni4 + nrb0 - 1) / nrb0 + 3) & ~3;
     int TC = (RB_THREADS / (TR / 4)) * 4;  // every thread owns a 4×4 block
     if (TC > 128) TC = 128;
-    if ((TC + 4) * 16 + TR * 16 > (int)(RB_TILE_DOUBLES * sizeof(double) / sizeof(T))) TC = 64;
     const int nrb = (a.ni + TR - 1) / TR;
     const long long ncb = (a.ncol + TC - 1) / TC;
-    const int nk = a.nk, nkt = a.B ? 2 * a.nk : a.nk;
-    // padded row of the column panel (16 bytes more in FP64, 16 in FP32): the transposing
-    // stores spread over the banks and every 4-column block stays 16-byte aligned
-    const int TCP = TC + (sizeof(T) == 8 ? 2 : 4);
-    T *As = reinterpret_cast<T *>(gs.tile), *Xs = As + KC * TR;
+    const int nk = a.nk;
+    const int TCP = TC + 4;  // padded row of the column panel: 4-column blocks stay 16-byte aligned
+    float *As = reinterpret_cast<float *>(gs.tile), *Xs = As + KC * TR;
     const int ib = threadIdx.x % (TR / 4), cb = threadIdx.x / (TR / 4);
     const bool owner = cb < TC / 4;
+    const int xk = threadIdx.x % KC, xc = threadIdx.x / KC;  // this thread's k of a panel, first column of a tile
+    int ai[EA], ak[EA];                                      // its operator elements: row of a tile, k of a panel
+#pragma unroll
+    for (int u = 0; u < EA; u++) {
+        const int e = threadIdx.x + u * RB_THREADS;
+        ak[u] = e / TR;
+        ai[u] = e - ak[u] * TR;
+    }
     for (long long tl = t.crank; tl < (long long)nrb * ncb; tl += t.ncta) {
-        const int i0 = (int)(tl % nrb) * TR;
-        const long long c0 = (tl / nrb) * TC;
-        constexpr bool SPLIT = sizeof(T) < 8;
-        T acc[4][4], accb[SPLIT ? 4 : 1][SPLIT ? 4 : 1];
+        const int i0 = nrb == 1 ? 0 : (int)(tl % nrb) * TR;
+        const long long c0 = (nrb == 1 ? tl : tl / nrb) * TC;
+        const TX *xp = a.X + a.ldx * c0;
+        int m[EX];
+        bool cok[EX];
+#pragma unroll
+        for (int u = 0; u < EX; u++) {
+            const int c = xc + u * (RB_THREADS / KC);
+            cok[u] = c < TC && c0 + c < a.ncol;
+            m[u] = 0;
+            if (sc.ys && cok[u]) m[u] = sc.mat[sc.nm == 1 ? c0 + c : (long long)((unsigned)(c0 + c) / (unsigned)sc.nm)];
+        }
+        float acc[4][4], accb[4][4];
 #pragma unroll
         for (int x = 0; x < 4; x++)
 #pragma unroll
-            for (int y = 0; y < 4; y++) acc[x][y] = T(0);
-        if (SPLIT)
-#pragma unroll
-            for (int x = 0; x < 4; x++)
-#pragma unroll
-                for (int y = 0; y < 4; y++) accb[SPLIT ? x : 0][SPLIT ? y : 0] = T(0);
-        // panels of the A part cover k < nk, those of the B part start at nk
+            for (int y = 0; y < 4; y++) acc[x][y] = accb[x][y] = 0.0f;
+        // panels of the A part first, then those of the B part
         const int npa = (nk + KC - 1) / KC, npanel = a.B ? 2 * npa : npa;
         for (int ip = 0; ip < npanel; ip++) {
             const bool partb = ip >= npa;
-            const int k0 = partb ? nk + (ip - npa) * KC : ip * KC;
-            const int kend = partb ? nkt : nk;
+            const int k0 = (partb ? ip - npa : ip) * KC;
+            const double *op = partb ? a.B : a.A;
             // every load of the panel is issued before the first shared-memory store
             double av[EA], xv[EX], sv[EX];
 #pragma unroll
             for (int u = 0; u < EA; u++) {
-                const int e = threadIdx.x + u * RB_THREADS;
-                const int i = i0 + e % TR, k = k0 + e / TR;
-                const bool in = e < KC * TR && i < a.ni && k < kend;
-                const double *op = k < nk ? a.A : a.B;
-                av[u] = in ? op[i + (long long)a.lda * (k < nk ? k : k - nk)] : 0.0;
+                const bool in = ak[u] < KC && i0 + ai[u] < a.ni && k0 + ak[u] < nk;
+                av[u] = in ? op[i0 + ai[u] + (long long)a.lda * (k0 + ak[u])] : 0.0;
             }
+            const int k = k0 + xk;
 #pragma unroll
             for (int u = 0; u < EX; u++) {
-                const int e = threadIdx.x + u * RB_THREADS;
-                const int k = k0 + e % KC;
-                const long long col = c0 + e / KC;
-                const bool in = e < KC * TC && k < kend && col < a.ncol;
-                xv[u] = in ? (double)a.X[(k < nk ? k : k - nk) * a.sx + a.ldx * col] : 0.0;
-                sv[u] = in ? scale(k, col) : 0.0;
+                const bool in = cok[u] && k < nk;
+                xv[u] = in ? (double)xp[k * a.sx + a.ldx * (xc + u * (RB_THREADS / KC))] : 0.0;
+                sv[u] = in ? (sc.ys ? (partb ? sc.tg[m[u]] : sc.ys[(long long)m[u] * nk + k]) : 1.0) : 0.0;
             }
             __syncthreads();
 #pragma unroll
-            for (int u = 0; u < EA; u++) {
-                const int e = threadIdx.x + u * RB_THREADS;
-                if (e < KC * TR) As[e] = (T)av[u];
-            }
+            for (int u = 0; u < EA; u++)
+                if (ak[u] < KC) As[threadIdx.x + u * RB_THREADS] = (float)av[u];
 #pragma unroll
             for (int u = 0; u < EX; u++) {
-                const int e = threadIdx.x + u * RB_THREADS;
-                if (e < KC * TC) Xs[(e % KC) * TCP + e / KC] = (T)(sv[u] * xv[u]);
+                const int c = xc + u * (RB_THREADS / KC);
+                if (c < TC) Xs[xk * TCP + c] = (float)(sv[u] * xv[u]);
             }
             __syncthreads();
             if (owner) {
+                auto block = [&](float (&s)[4][4]) {
 #pragma unroll 4
-                for (int kk = 0; kk < KC; kk++) {
-                    T o[4], v[4];
-                    Vec4<T>::load(As + kk * TR + ib * 4, o);
-                    Vec4<T>::load(Xs + kk * TCP + cb * 4, v);
-                    if (SPLIT && partb) {
+                    for (int kk = 0; kk < KC; kk++) {
+                        const float4 o4 = *reinterpret_cast<const float4 *>(As + kk * TR + ib * 4);
+                        const float4 v4 = *reinterpret_cast<const float4 *>(Xs + kk * TCP + cb * 4);
+                        const float o[4] = {o4.x, o4.y, o4.z, o4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
                         for (int x = 0; x < 4; x++)
 #pragma unroll
-                            for (int y = 0; y < 4; y++) accb[SPLIT ? x : 0][SPLIT ? y : 0] += o[x] * v[y];
-                    } else {
-#pragma unroll
-                        for (int x = 0; x < 4; x++)
-#pragma unroll
-                            for (int y = 0; y < 4; y++) acc[x][y] += o[x] * v[y];
+                            for (int y = 0; y < 4; y++) s[x][y] += o[x] * v[y];
                     }
-                }
+                };
+                if (partb) block(accb);
+                else block(acc);
             }
         }
         if (owner) {  // epilogue: the loads `pre` makes for the 16 outputs first, then the stores
@@ -772,9 +761,7 @@ __device__ void team_product(Team &t, GroupShared &gs, const ProductArgs<TX> &a,
 #pragma unroll
                 for (int x = 0; x < 4; x++) {
                     const int i = i0 + ib * 4 + x;
-                    if (i < a.ni)
-                        store(i, col, SPLIT ? (double)acc[x][y] + (double)accb[SPLIT ? x : 0][SPLIT ? y : 0] : (double)acc[x][y],
-                              pv[x][y]);
+                    if (i < a.ni) store(i, col, (double)acc[x][y] + (double)accb[x][y], pv[x][y]);
                 }
             }
         }
@@ -795,13 +782,9 @@ __device__ void m2d_tiles(Team &t, const DevProblem &P, GroupShared &gs, void *r
     const double *ys = P.kmat;
     if (mixed && scaled) {
         ProductArgs<double> a{P.mn, P.mnfp, nd, nd, np, src, 1, np, ncol};
-        auto sc = [=, &gs] __device__(int k, long long col) {
-            const int m = mat[col / nm];
-            return k < np ? ys[(long long)m * np + k] : gs.tg[m];
-        };
         auto pre = [=] __device__(int i, long long col) { return add ? add[col * sc_ + i * sn] : 0.0; };
         float *psi = P.psi32;
-        team_product<float>(t, gs, a, sc, pre, [=] __device__(int i, long long col, double v, double ad) {
+        product32(t, gs, a, Scale32{ys, gs.tg, mat, nm}, pre, [=] __device__(int i, long long col, double v, double ad) {
             psi[col * sc_ + i * sn] = (float)(ad + v);
         });
         return;
@@ -820,11 +803,10 @@ __device__ void d2m_tiles(Team &t, const DevProblem &P, GroupShared &gs, void *r
     const int nd = P.nd, np = P.np, nm = P.nm5;
     const long long ncol = (long long)nm * P.ncell;
     if (mixed) {
-        auto one = [] __device__(int, long long) { return 1.0; };
         auto pre = [=] __device__(int i, long long col) { return matvec ? zin[col * np + i] : 0.0; };
         auto st = [=] __device__(int i, long long col, double v, double z) { zout[col * np + i] = matvec ? z - v : v; };
         ProductArgs<float> a{P.dn, nullptr, np, np, nd, P.psi32, P.psi_sn, P.psi_sc, ncol};
-        team_product<float>(t, gs, a, one, pre, st);
+        product32(t, gs, a, Scale32{nullptr, nullptr, nullptr, 1}, pre, st);
         return;
     }
     Prod64 a{P.dn, nullptr, np, 1, np, nd, P.psi, P.psi_sn, P.psi_sc, ncol, nullptr, 0, nullptr, P.mat, nm,

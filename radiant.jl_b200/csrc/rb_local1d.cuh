@@ -25,7 +25,7 @@ namespace rb {
 #define RB_LMAP (RB_SCAN_NF * RB_SCAN_NF + RB_SCAN_NF)  // doubles of one face map
 #define RB_LKEYS 2  // distinct (material, width) cell kinds per CTA with factored cell operators
 
-// a CTA-local team: team_product over this CTA's columns only
+// a CTA-local team: products over this CTA's columns only
 struct CtaTeam {
     unsigned crank = 0, ncta = 1;
 };
@@ -569,7 +569,7 @@ __device__ bool sweep1d_local_fixed(ClusterTeam &t, const DevProblem &P, GroupSh
 
 // the products of the local pass, compiled as functions of their own so that their registers
 // are allocated apart from the rest of the solve: FP64 on the FP64 tensor pipe (prod_tiles, the
-// operators resident where they fit), FP32 (mixed form) through team_product
+// operators resident where they fit), FP32 (mixed form) through product32
 template <typename T, typename PS>
 __device__ __noinline__ void m2d_local(const DevProblem &P, GroupShared &gs, Local1D &L, const double *zin,
                                        int homog) {
@@ -600,12 +600,8 @@ __device__ __noinline__ void m2d_local(const DevProblem &P, GroupShared &gs, Loc
             }
         } else {
             ProductArgs<double> a{P.mn, P.mnfp, nd, nd, np, zin + (long long)np * col0, 1, np, ncl};
-            auto sc = [=, &gs] __device__(int k, long long lc) {
-                const int m = mat[lc / nm];
-                return k < np ? ys[(long long)m * np + k] : gs.tg[m];
-            };
             auto pre = [=] __device__(int i, long long lc) { return add ? add[(col0 + lc) * nd + i] : 0.0; };
-            team_product<T>(ct, gs, a, sc, pre, [=] __device__(int i, long long lc, double v, double ad) {
+            product32(ct, gs, a, Scale32{ys, gs.tg, mat, nm}, pre, [=] __device__(int i, long long lc, double v, double ad) {
                 psi[i + ldp * lc] = (PS)(ad + v);
             });
         }
@@ -634,9 +630,8 @@ __device__ __noinline__ void d2m_local(const DevProblem &P, GroupShared &gs, Loc
             }
         } else {
             ProductArgs<PS> a{P.dn, nullptr, np, np, nd, psi, 1, ldp, ncl};
-            auto one = [] __device__(int, long long) { return 1.0; };
             auto pre = [=] __device__(int i, long long lc) { return matvec ? zin[(col0 + lc) * np + i] : 0.0; };
-            team_product<T>(ct, gs, a, one, pre, [=] __device__(int i, long long lc, double v, double z) {
+            product32(ct, gs, a, Scale32{nullptr, nullptr, nullptr, 1}, pre, [=] __device__(int i, long long lc, double v, double z) {
                 zout[(col0 + lc) * np + i] = matvec ? z - v : v;
             });
         }

@@ -3,7 +3,7 @@
 //
 // The products are the M2D and D2M lines of sn_sweep_2D.jl:54-183 / sn_sweep_3D.jl:57-239
 // (Qn = Mn[n,:]·Ql, 𝚽l += Dn[:,n]·𝚽n) with the in-group scattering (scattering_source.jl:25-30)
-// and Fokker-Planck (fokker_planck_source.jl:29-33) sources folded in, as team_product does in
+// and Fokker-Planck (fokker_planck_source.jl:29-33) sources folded in, as prod64_team does in
 // FP64 (rb_kernels.cuh):
 //   M2D  ψ[col,n] = pre + Σ_p ys[mat,p]·𝚽[col,p]·Mn[n,p] + Σ_p T[mat]·𝚽[col,p]·(Mn·ℳ)[n,p]
 //   D2M  z[col,p] = pre ∓ Σ_n ψ[col,n]·Dn[p,n]
@@ -299,7 +299,7 @@ __device__ bool tc_product(Team &t, TcState &ts, unsigned char *sm, long long sm
 }
 
 // The M2D product of a mixed-form 2D/3D pass on the tensor cores (into the FP32 angular buffer);
-// false when the shapes do not fit (the caller then uses team_product).
+// false when the shapes do not fit (the caller then uses product32).
 template <class Team>
 __device__ bool m2d_tc(Team &t, const DevProblem &P, GroupShared &gs, TcState &ts, void *smem, long long smem_bytes,
                        const double *zin, const double *add) {
