@@ -88,7 +88,7 @@ template <typename R>
 struct Oct3dSmem {
     static constexpr long long DB = OctDB<R>::value, T = RB_OCT_TILE, TP = T * T;
     static constexpr long long RS = (long long)sizeof(R);
-    static constexpr int DC = sizeof(R) == 8 ? 10 : 12;                      // constants per direction, padded to 16 bytes
+    static constexpr int DC = sizeof(R) == 8 ? 6 : 8;                        // constants per direction, padded to 16 bytes
     static constexpr long long CS = DB % 4 == 2 ? DB : DB + 2;               // widest cell stride of a stage (below)
     static constexpr int MROW = RB_OCT_MATNX + 4;                            // bytes of a pencil's materials
     static constexpr long long al(long long b) { return (b + 15) & ~15LL; }
@@ -96,7 +96,8 @@ struct Oct3dSmem {
     static constexpr long long fz = fy + al(2 * T * DB * 8);                // double [2][T][DB]
     static constexpr long long dc = fz + al(2 * T * DB * 8);                // R [DB][DC]
     static constexpr long long sfz = dc + al(DB * DC * RS);                 // R [2][DB][TP]
-    static constexpr long long qb = sfz + al(2 * DB * TP * RS);             // R [2][TP][CS]
+    static constexpr long long yo = sfz + al(2 * DB * TP * RS);             // R [2][DB][T] y faces leaving the tile
+    static constexpr long long qb = yo + al(2 * DB * T * RS);               // R [2][TP][CS]
     static constexpr long long ix = qb + al(2 * CS * TP * RS);              // R [RB_OCT_MAXNX]
     static constexpr long long ms = ix + al(RB_OCT_MAXNX * RS);             // R [RB_MAXMAT]
     static constexpr long long mq = ms + al(RB_MAXMAT * RS);                // R [RB_MAXMAT]
@@ -165,9 +166,11 @@ __device__ __forceinline__ bool wait_progress(const unsigned long long *f, unsig
 // on the IBM RISC System/6000 processor", 1990) without a branch, so the chains of a cell's
 // directions interleave; the divide instruction sequence ends each one in a branch. Operands
 // outside the range where the correction is exact take the divide.
-__device__ __forceinline__ double oct_div(double q, double s) {
+__device__ __forceinline__ bool oct_div_range(double s) {
     const double a = fabs(s);
-    if (!(a > 1e-140 && a < 1e140)) return q / s;
+    return a > 1e-140 && a < 1e140;
+}
+__device__ __forceinline__ double oct_div_fast(double q, double s) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
     r = fma(r, fma(-s, r, 1.0), r);
@@ -175,7 +178,24 @@ __device__ __forceinline__ double oct_div(double q, double s) {
     const double v = q * r;
     return fma(fma(-s, v, q), r, v);
 }
-__device__ __forceinline__ float oct_div(float q, float s) { return __fdividef(q, s); }
+__device__ __forceinline__ double oct_div(double q, double s) { return oct_div_range(s) ? oct_div_fast(q, s) : q / s; }
+__device__ __forceinline__ bool oct_div_range(float) { return true; }
+__device__ __forceinline__ float oct_div_fast(float q, float s) { return __fdividef(q, s); }
+
+// the six constants of a direction, as 16-byte loads
+__device__ __forceinline__ void load6(double (&d)[6], const double *p) {
+#pragma unroll
+    for (int i = 0; i < 6; i += 2) {
+        const double2 x = *reinterpret_cast<const double2 *>(p + i);
+        d[i] = x.x;
+        d[i + 1] = x.y;
+    }
+}
+__device__ __forceinline__ void load6(float (&d)[6], const float *p) {
+    const float4 x = *reinterpret_cast<const float4 *>(p);
+    const float2 y = *reinterpret_cast<const float2 *>(p + 4);
+    d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w; d[4] = y.x; d[5] = y.y;
+}
 
 template <typename T> struct Pair;
 template <> struct Pair<float> { using type = float2; };
@@ -220,7 +240,7 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
     double *fyb = reinterpret_cast<double *>(base + L::fy);
     double *fzb = reinterpret_cast<double *>(base + L::fz);
     R *dc = reinterpret_cast<R *>(base + L::dc);
-    R *sfz = reinterpret_cast<R *>(base + L::sfz);
+    R *sfz = reinterpret_cast<R *>(base + L::sfz), *yo = reinterpret_cast<R *>(base + L::yo);
     R *idxs = reinterpret_cast<R *>(base + L::ix);
     R *mS = reinterpret_cast<R *>(base + L::ms);
     R *mQ = reinterpret_cast<R *>(base + L::mq);
@@ -277,14 +297,20 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                 const double ac = RECIP ? 1.0 : (me < cnt ? fabs(P.cosv[(long long)a * nd + n]) : 0.0);
                 dc[me * DC + a] = me < cnt ? (R)(ac * P.G[blk]) : R(0);
                 dc[me * DC + 3 + a] = me < cnt ? (R)(ac * P.Gsrc[blk * nfm]) : R(0);
-                dc[me * DC + 6 + a] = me < cnt ? (R)P.Gout[blk * nfm] : R(0);
             }
         }
+        // one-moment cells: the face closure's coefficient does not depend on the direction
+        const R gox = (R)P.Gout[(long long)first * 3 * nfm], goy = (R)P.Gout[((long long)first * 3 + 1) * nfm];
+        const R goz = (R)P.Gout[((long long)first * 3 + 2) * nfm];
+        // the last pencils of the tile, whose faces leave it
+        const int jyE = min(TY, ny - tyq * TY) - 1, jzE = min(TZ, nz - tzq * TZ) - 1;
         // The faces entering the tile in a step, one direction of one pencil per item: pencils
         // (0, j) for y faces, then (j, 0) for z faces; a thread has up to RB_OCT_ITEMS of them.
         constexpr int NI = (2 * TT * DB + TP - 1) / TP;
         const double *isrc[NI];  // the item's face at x column 0
+        double *iout[NI];        // and the same item's face leaving the tile, from its last pencils
         int ij[NI], idst[NI];    // its pencil's offset in steps (−1: none) and place in a stage
+        int io[NI], iv[NI];      // the leaving face's offset in steps and place in yo (≥ 0) or sfz (−1 − place)
         {
             const int nfy = TZ * cnt, nfz = TY * cnt;
 #pragma unroll
@@ -292,6 +318,8 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                 const int e = me + u * TP;
                 ij[u] = -1;
                 isrc[u] = nullptr;
+                iout[u] = nullptr;
+                io[u] = iv[u] = 0;
                 idst[u] = 0;
                 if (e < nfy + nfz) {
                     const bool isy = e < nfy;
@@ -302,6 +330,10 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                         const long long off = isy ? (tyq == 0 ? yin : yoff) : (tzq == 0 ? zin_ : zoff);
                         isrc[u] = fexit + (long long)(first + kk) * sstride + off + (long long)nx * row * nfm;
                         ij[u] = j;
+                        const long long out = isy ? (tyq == nty - 1 ? eyo : yoff) : (tzq == ntz - 1 ? ezo : zoff);
+                        iout[u] = fexit + (long long)(first + kk) * sstride + out + (long long)nx * row * nfm;
+                        io[u] = j + (isy ? jyE : jzE);
+                        iv[u] = isy ? kk * TT + j : -1 - (kk * TP + jzE * TY + j);
                         idst[u] = (isy ? 0 : (int)((L::fz - L::fy) / 8)) + j * LDB + kk;
                     }
                 }
@@ -328,6 +360,18 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                 }
             }
             cp_async_commit();
+        };
+        // the faces that step s left to the downstream tiles (or the domain), an item per thread
+        auto store_faces = [&](int s) {
+            const int b = s & 1;
+#pragma unroll
+            for (int u = 0; u < NI; u++) {
+                const int ixx = s - io[u];
+                if (ij[u] >= 0 && ixx >= 0 && ixx < nx) {
+                    const R f = iv[u] >= 0 ? yo[b * LDB * TT + iv[u]] : sfz[b * LDB * TP - 1 - iv[u]];
+                    iout[u][(long long)(fx ? ixx : nx - 1 - ixx) * nfm] = (double)f;
+                }
+            }
         };
         const R idy = pok ? (R)(1.0 / P.dy[iy]) : R(0), idz = pok ? (R)(1.0 / P.dz[iz]) : R(0);
         const unsigned c0 = (unsigned)nx * (iy + ny * iz);  // the pencil's first cell
@@ -405,10 +449,11 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
             wait_up(sg + 1);
             cp_async_wait<0>();  // this thread's copies of step sg have landed
             __syncthreads();     // everyone's; step sg − 1 solved; step sg + 1's faces are written
-            // steps < sg are done: publish (the barrier orders every thread's face stores before the
-            // release), by another warp than the one that waits for the upwind tiles
-            if (me == RB_OCT_PUBLISHER && sg > 0 && sg % RB_OCT_PUB == 0)
-                st_release_u64(flags + t.crank, tagr | (unsigned long long)sg);
+            // the faces of steps < sg − 1 are stored: publish (the barrier orders every thread's stores
+            // before the release), by another warp than the one that waits for the upwind tiles
+            if (me == RB_OCT_PUBLISHER && sg > 1 && (sg - 1) % RB_OCT_PUB == 0)
+                st_release_u64(flags + t.crank, tagr | (unsigned long long)(sg - 1));
+            if (sg > 0) store_faces(sg - 1);
             if (sg + 1 < nsteps) stage_cells(sg + 1);
             stage_faces(sg + 1);
             const int ixx = sg - dstep;
@@ -460,7 +505,8 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
 #pragma unroll
                     for (int k = 0; k < DB; k++) {
                         if (k >= cnt) continue;
-                        const R *d = dc + k * DC;
+                        R d[6];
+                        load6(d, dc + k * DC);
                         const int n = first + k;
                         const R hx = oct_div(fabs(P.cosv[n]), P.dx[ix]), hy = oct_div(fabs(P.cosv[nd + n]), P.dy[iy]);
                         const R hz = oct_div(fabs(P.cosv[2 * nd + n]), P.dz[iz]);
@@ -472,21 +518,37 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                         q += hy * (d[4] * fyi[k]);
                         q += hz * (d[5] * fzi[k]);
                         v[k] = q * oct_div(1.0, S);
-                        fxs[k] = w1x * fxs[k] + d[6] * v[k];
-                        fyi[k] = w1y * fyi[k] + d[7] * v[k];
-                        fzi[k] = w1z * fzi[k] + d[8] * v[k];
+                        fxs[k] = w1x * fxs[k] + gox * v[k];
+                        fyi[k] = w1y * fyi[k] + goy * v[k];
+                        fzi[k] = w1z * fzi[k] + goz * v[k];
                     }
                 } else {
+                    // every direction's collision term and right-hand side, then the quotients, then the
+                    // faces: three loops without a branch, so that the directions' chains overlap
+                    R S[DB];
+                    bool fast = true;
 #pragma unroll
                     for (int k = 0; k < DB; k++) {
-                        const R *d = dc + k * DC;
-                        const R S = S0 + d[0] * idx + d[1] * idy + d[2] * idz;
+                        R d[6];
+                        load6(d, dc + k * DC);
+                        S[k] = S0 + d[0] * idx + d[1] * idy + d[2] * idz;
                         R q = v[k] + (d[3] * idx) * fxs[k] + (d[4] * idy) * fyi[k] + (d[5] * idz) * fzi[k];
                         if (CSD) q -= sq * fe[CSD ? k : 0];
-                        v[k] = oct_div(q, S);
-                        fxs[k] = w1x * fxs[k] + d[6] * v[k];
-                        fyi[k] = w1y * fyi[k] + d[7] * v[k];
-                        fzi[k] = w1z * fzi[k] + d[8] * v[k];
+                        v[k] = q;
+                        fast = fast && oct_div_range(S[k]);
+                    }
+                    if (fast) {
+#pragma unroll
+                        for (int k = 0; k < DB; k++) v[k] = oct_div_fast(v[k], S[k]);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < DB; k++) v[k] = v[k] / S[k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < DB; k++) {
+                        fxs[k] = w1x * fxs[k] + gox * v[k];
+                        fyi[k] = w1y * fyi[k] + goy * v[k];
+                        fzi[k] = w1z * fzi[k] + goz * v[k];
                     }
                 }
 #pragma unroll
@@ -510,24 +572,10 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                         if (CSD) ec[k] = (double)(w1e * fe[CSD ? k : 0] + eout * v[k]);
                     }
                 }
-                // faces leaving the tile or the domain
-                if (jy == TY - 1 || iyy == ny - 1) {
-                    double *f = fexit + (long long)first * sstride + (iyy < ny - 1 ? yoff : eyo) + (ix + (long long)nx * iz) * nfm;
+                if (jy == jyE) {  // (the z faces are in sfz)
 #pragma unroll
                     for (int k = 0; k < DB; k++)
-                        if (k < cnt) f[(long long)k * sstride] = (double)fyi[k];
-                }
-                if (jz == TZ - 1 || izz == nz - 1) {
-                    double *f = fexit + (long long)first * sstride + (izz < nz - 1 ? zoff : ezo) + (ix + (long long)nx * iy) * nfm;
-#pragma unroll
-                    for (int k = 0; k < DB; k++)
-                        if (k < cnt) f[(long long)k * sstride] = (double)fzi[k];
-                }
-                if (ixx == nx - 1) {
-                    double *f = fexit + (long long)first * sstride + (iy + (long long)ny * iz) * nfm;
-#pragma unroll
-                    for (int k = 0; k < DB; k++)
-                        if (k < cnt) f[(long long)k * sstride] = (double)fxs[k];
+                        if (k < cnt) yo[(wr * LDB + k) * TT + jz] = fyi[k];
                 }
             }
 #pragma unroll
@@ -537,6 +585,14 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
             __syncwarp();  // before the stage takes the step after the next
         }
         cp_async_wait<0>();
+        __syncthreads();
+        store_faces(nsteps - 1);
+        if (pok) {  // the x faces leaving the domain
+            double *f = fexit + (long long)first * sstride + (iy + (long long)ny * iz) * nfm;
+#pragma unroll
+            for (int k = 0; k < DB; k++)
+                if (k < cnt) f[(long long)k * sstride] = (double)fxs[k];
+        }
         __syncthreads();
         if (me == RB_OCT_PUBLISHER) st_release_u64(flags + t.crank, tagr | (unsigned long long)nsteps);
     }
