@@ -865,6 +865,7 @@ int launch_grid(rb_context *ctx, DevProblem *prob, const DevProblem &hp, cudaStr
         };
         need = std::max(need, std::max(plan(h.nd, h.np, parts), plan(h.np, h.nd, 1)));
     }
+    if (h.accel == RB_ACCEL_BICGSTAB) need = std::max(need, 20LL * RB_THREADS * 16);  // its streamed vector loops
     if (need > avail) need = 0;  // the problem then takes the paths that need no region
     const int local_bytes = (int)((need + 1023) & ~1023LL);
     const size_t smem = sizeof(rb::GroupShared) + local_bytes;

@@ -640,10 +640,58 @@ struct Solver {
         return st;
     }
 
+    // The vector loops of BiCGStab on the grid team: a thread's pairs come by cp.async into its own
+    // slots, several turns ahead, so that the reads of the loop's vectors stay in flight while it works
+    // (loops that load a batch of pairs and then use it drain the pipe at every turn: 2.6 TB/s at 64³
+    // with 256 threads a SM). Same pairs per thread and same order as RB_VPAIRS, so the same sums.
+    // f(pair index, x[NV]) for each pair; `local` is free between the phases of a pass.
+    template <int NV, class F>
+    __device__ __forceinline__ void stream(const double2 *const (&src)[NV], long long N2, F f) {
+        const long long q1 = N2 * (t.crank + 1) / t.ncta, q0 = N2 * t.crank / t.ncta + threadIdx.x;
+        constexpr int S = NV <= 2 ? 8 : (NV == 3 ? 6 : 4);  // turns in flight
+        double2 *slot = reinterpret_cast<double2 *>(local) + threadIdx.x;  // [S][NV][threads]
+        auto issue = [&](long long q, int s) {
+            if (q < q1)
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    cp_zfill<16>(reinterpret_cast<double *>(slot + (s * NV + v) * RB_THREADS),
+                                 reinterpret_cast<const double *>(src[v] + q), true);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll 1
+        for (int s = 0; s < S; s++) issue(q0 + s * RB_THREADS, s);
+        int s = 0;
+#pragma unroll 1
+        for (long long q = q0; q < q1; q += RB_THREADS) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(S - 1) : "memory");
+            double2 x[NV];
+#pragma unroll
+            for (int v = 0; v < NV; v++) x[v] = slot[(s * NV + v) * RB_THREADS];
+            issue(q + S * RB_THREADS, s);
+            s = s + 1 == S ? 0 : s + 1;
+            f(q, x);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    static constexpr long long stream_bytes = 20LL * RB_THREADS * 16;  // the largest S·NV
+    template <int NV, class F>
+    __device__ __forceinline__ void vloop(const double2 *const (&src)[NV], long long N2, F f) {
+        if constexpr (std::is_same<Team, GridTeam>::value) {
+            if (local_bytes >= stream_bytes) {
+                stream<NV>(src, N2, f);
+                return;
+            }
+        }
+        double2 xv[4][NV];
+        RB_VPAIRS_D(t, N2, 4, {
+#pragma unroll
+            for (int v = 0; v < NV; v++) xv[u_][v] = src[v][q];
+        }, { f(q, xv[u_]); })
+    }
+
     // ---------------------------------------------------------------- bicgstab
     // Vector loops over 16-byte element pairs of CTA-contiguous slices (the pad element of an odd
-    // state stays zero in every vector): 8 pairs in flight per thread over two vectors, 4 over
-    // three or four.
+    // state stays zero in every vector).
     __device__ __noinline__ SolveStat bicgstab(double *z, const double *rhs, int maxit, double tol) {
         const long long N = P.nstate, N2 = P.vstride / 2;
         SolveStat st = {0, 0.0, 1, CUDART_NAN};
@@ -655,15 +703,12 @@ struct Solver {
         const double2 zero2 = make_double2(0.0, 0.0);
         matvec(r, z);
         double a1[1] = {0.0};
-        {
-            double2 xc[RB_VU2], xr[RB_VU2];
-            RB_VPAIRS(t, N2, { xc[u_] = c2[q]; xr[u_] = r2[q]; }, {
-                const double2 ri = make_double2(xc[u_].x - xr[u_].x, xc[u_].y - xr[u_].y);
-                r2[q] = ri; rh2[q] = ri; p2[q] = zero2; v2[q] = zero2;
-                a1[0] += ri.x * ri.x;
-                a1[0] += ri.y * ri.y;
-            })
-        }
+        vloop<2>({c2, r2}, N2, [&](long long q, const double2 (&x)[2]) {
+            const double2 ri = make_double2(x[0].x - x[1].x, x[0].y - x[1].y);
+            r2[q] = ri; rh2[q] = ri; p2[q] = zero2; v2[q] = zero2;
+            a1[0] += ri.x * ri.x;
+            a1[0] += ri.y * ri.y;
+        });
         t.template sumk<1>(a1);
         int iter = 1, conv = 0;
         double resid = sqrt(a1[0]) / bnorm, resid0 = resid;
@@ -677,28 +722,28 @@ struct Solver {
             const double rho_new = rho_next;
             if (fabs(rho_new) < tiny) break;
             const double beta = (rho_new / rho_old) * (alpha / omega);
-            {
-                double2 xr[4], xp[4], xv[4];
-                RB_VPAIRS_D(t, N2, 4, { xr[u_] = r2[q]; xp[u_] = p2[q]; xv[u_] = v2[q]; }, {
-                    p2[q] = make_double2(xr[u_].x + 1.0 * (beta * (xp[u_].x + (-omega) * xv[u_].x)),
-                                         xr[u_].y + 1.0 * (beta * (xp[u_].y + (-omega) * xv[u_].y)));
-                })
-            }
+            vloop<3>({r2, p2, v2}, N2, [&](long long q, const double2 (&x)[3]) {
+                p2[q] = make_double2(x[0].x + 1.0 * (beta * (x[1].x + (-omega) * x[2].x)),
+                                     x[0].y + 1.0 * (beta * (x[1].y + (-omega) * x[2].y)));
+            });
             t.sync();
             matvec(v, p); iter++;
-            const double denom = vdot2(t, rh, v, N2);
+            double a0[1] = {0.0};
+            vloop<2>({rh2, v2}, N2, [&](long long, const double2 (&x)[2]) {
+                a0[0] += x[0].x * x[1].x;
+                a0[0] += x[0].y * x[1].y;
+            });
+            t.template sumk<1>(a0);
+            const double denom = a0[0];
             if (fabs(denom) < tiny) break;
             alpha = rho_new / denom;
             double a2[1] = {0.0};
-            {
-                double2 xr[RB_VU2], xv[RB_VU2];
-                RB_VPAIRS(t, N2, { xr[u_] = r2[q]; xv[u_] = v2[q]; }, {
-                    const double2 si = make_double2(xr[u_].x + (-alpha) * xv[u_].x, xr[u_].y + (-alpha) * xv[u_].y);
-                    s2[q] = si;
-                    a2[0] += si.x * si.x;
-                    a2[0] += si.y * si.y;
-                })
-            }
+            vloop<2>({r2, v2}, N2, [&](long long q, const double2 (&x)[2]) {
+                const double2 si = make_double2(x[0].x + (-alpha) * x[1].x, x[0].y + (-alpha) * x[1].y);
+                s2[q] = si;
+                a2[0] += si.x * si.x;
+                a2[0] += si.y * si.y;
+            });
             t.template sumk<1>(a2);
             const double sn_ = sqrt(a2[0]);
             if (sn_ / bnorm < tol) {
@@ -709,32 +754,25 @@ struct Solver {
             }
             matvec(tt, s); iter++;
             double a3[2] = {0.0, 0.0};
-            {
-                double2 xt[RB_VU2], xs[RB_VU2];
-                RB_VPAIRS(t, N2, { xt[u_] = t2[q]; xs[u_] = s2[q]; }, {
-                    a3[0] += xt[u_].x * xt[u_].x;
-                    a3[0] += xt[u_].y * xt[u_].y;
-                    a3[1] += xt[u_].x * xs[u_].x;
-                    a3[1] += xt[u_].y * xs[u_].y;
-                })
-            }
+            vloop<2>({t2, s2}, N2, [&](long long, const double2 (&x)[2]) {
+                a3[0] += x[0].x * x[0].x;
+                a3[0] += x[0].y * x[0].y;
+                a3[1] += x[0].x * x[1].x;
+                a3[1] += x[0].y * x[1].y;
+            });
             t.template sumk<2>(a3);
             if (a3[0] < tiny) break;
             omega = a3[1] / a3[0];
             double a4[2] = {0.0, 0.0};
-            {
-                double2 xz[4], xp[4], xs[4], xt[4], xh[4];
-                RB_VPAIRS_D(t, N2, 4, { xz[u_] = z2[q]; xp[u_] = p2[q]; xs[u_] = s2[q]; xt[u_] = t2[q]; xh[u_] = rh2[q]; }, {
-                    z2[q] = make_double2((xz[u_].x + alpha * xp[u_].x) + omega * xs[u_].x,
-                                         (xz[u_].y + alpha * xp[u_].y) + omega * xs[u_].y);
-                    const double2 ri = make_double2(xs[u_].x + (-omega) * xt[u_].x, xs[u_].y + (-omega) * xt[u_].y);
-                    r2[q] = ri;
-                    a4[0] += ri.x * ri.x;
-                    a4[0] += ri.y * ri.y;
-                    a4[1] += xh[u_].x * ri.x;
-                    a4[1] += xh[u_].y * ri.y;
-                })
-            }
+            vloop<5>({z2, p2, s2, t2, rh2}, N2, [&](long long q, const double2 (&x)[5]) {
+                z2[q] = make_double2((x[0].x + alpha * x[1].x) + omega * x[2].x, (x[0].y + alpha * x[1].y) + omega * x[2].y);
+                const double2 ri = make_double2(x[2].x + (-omega) * x[3].x, x[2].y + (-omega) * x[3].y);
+                r2[q] = ri;
+                a4[0] += ri.x * ri.x;
+                a4[0] += ri.y * ri.y;
+                a4[1] += x[4].x * ri.x;
+                a4[1] += x[4].y * ri.y;
+            });
             t.template sumk<2>(a4);
             rho_next = a4[1];
             resid = sqrt(a4[0]) / bnorm;
