@@ -791,6 +791,7 @@ __device__ void m2d_tiles(Team &t, const DevProblem &P, GroupShared &gs, void *r
     }
     Prod64 a{P.mn, scaled ? P.mnfp : nullptr, nd, 1, nd, np, src, 1, np, ncol,
              scaled ? ys : nullptr, np, (scaled && P.mnfp) ? gs.tg : nullptr, mat, nm, add, 1.0, out, sn, sc_};
+    a.interleave = P.precision == 0;
     const bool own = bytes >= (long long)sizeof(gs.tile);
     prod64_team(t, a, own ? region : (void *)gs.tile, own ? bytes : (long long)sizeof(gs.tile));
 }

@@ -592,6 +592,7 @@ __device__ __noinline__ void m2d_local(const DevProblem &P, GroupShared &gs, Loc
             if (add) __syncthreads();
             Prod64 a{P.mn, P.mnfp, nd, 1, nd, np, zin + (long long)np * col0, 1, np, ncl, ys, np,
                      P.mnfp ? gs.tg : nullptr, mat, nm, add ? psi : nullptr, 1.0, psi, 1, ldp};
+            a.interleave = P.precision == 0;
             if (L.opM) {
                 prod_run(a, L.opM, 0, prod_nt(nd), threadIdx.x >> 5, blockDim.x >> 5);
                 __syncthreads();

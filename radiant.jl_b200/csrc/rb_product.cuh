@@ -44,6 +44,9 @@ struct Prod64 {
     // operator columns are zero); else n is i (the others' outputs are left alone). null: all.
     const double *sel = nullptr;
     bool selk = false, selpos = false;
+    // both parts on a piece of k before the next piece (the columns are loaded once, not twice): the
+    // plain form. The mixed form, whose FP32 roundings follow the last bit, keeps part A before B.
+    bool interleave = false;
 };
 
 #define RB_PROD_MAXNT 12  // row tiles (of 8) a warp accumulates at once
@@ -120,11 +123,13 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
     const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
     constexpr int LD = 8 * NT + 4;
     constexpr int CH = NT * MT >= 16 ? 4 : 8;  // k-steps (of 4) of a column loaded ahead, by the registers left
-    // k runs through part A, then part B: one accumulator takes the terms in the order of a plain
-    // loop over k (the MMA itself adds its four products in order, each rounded: an FMA chain)
+    // one accumulator takes the terms in the order of a plain loop over k (the MMA itself adds its
+    // four products in order, each rounded: an FMA chain), through part A, then part B, or piece by
+    // piece of both
     const int kp = prod_kp(a.nk), nks = kp / 4, npc = (nks + CH - 1) / CH;
     const bool two = a.B != nullptr;
-    const int nch = two ? 2 * npc : npc;
+    const bool inter = two && a.interleave;
+    const int nch = two && !inter ? 2 * npc : npc;
     const uint32_t ob = (uint32_t)__cvta_generic_to_shared(op) + (uint32_t)(q * LD + r) * 8;
     const long long ngrp = (a.ncol + 8 * MT - 1) / (8 * MT);
     if (w0 >= ngrp) return;
@@ -191,6 +196,16 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
                         const double b = lds64(o + n * 64);
 #pragma unroll
                         for (int mt = 0; mt < MT; mt++) dmma(acc[mt][n], av[mt], b);
+                    }
+                    if (inter) {
+#pragma unroll
+                        for (int mt = 0; mt < MT; mt++) av[mt] = tq[mt] * xc[mt][u];
+#pragma unroll
+                        for (int n = 0; n < NT; n++) {
+                            const double b = lds64(o + (uint32_t)kp * (LD * 8) + n * 64);
+#pragma unroll
+                            for (int mt = 0; mt < MT; mt++) dmma(acc[mt][n], av[mt], b);
+                        }
                     }
                 }
             }
