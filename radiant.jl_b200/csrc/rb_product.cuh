@@ -19,7 +19,9 @@
 // block r mod nrb), which reads the columns nrb times but never reloads the operator.
 //
 // What bounds it: the 3D products stream z and ψ (HBM and L2), the 2D ones with their 168
-// directions the FP64 pipe (5.25 flops per byte of L2 traffic and element).
+// directions the FP64 pipe, the 1D ones the latency of a call. M2D of 48×41×35 cells, S8, two parts:
+// 350 us as staged panels on the FP64 cores, 116 here; 128×128, S12: 203 and 90; 152 columns of a
+// slab team, 32 rows, two parts: 35 and 14.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -214,7 +214,7 @@ template <> struct Pair<double> { using type = double2; };
 // load, so a warp's 32 cells are staged together, cnt / VW neighbouring lanes on the run of one
 // cell, with each lane's pencils and offsets worked out once per task; the same lanes write the
 // results back. VW = 2: the batch's directions start and count even (pairs). Sweep at 64³, S8,
-// mixed: 2070 us (element-wise staging, addresses per element), 1030 (each thread its own cell).
+// mixed: 2070 us (element-wise staging, addresses per element), 1030 (each thread its own cell), 960 now.
 // RECIP: the cell as sweep_3d_tiles solves it (DevProblem::recip).
 template <typename R, int DB, int VW, bool CSD, bool RECIP, class Team>
 __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShared &gs, void *smem,
@@ -441,6 +441,21 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                 fxs[k] = (pok && k < cnt) ? (R)fexit[(long long)(first + k) * sstride + o] : R(0);
             }
         }
+        // RECIP: h = |Ω|/Δ per axis, the pencil's y and z ones once, the x ones where the width changes
+        // (dxn: the next cell's width, loaded a step ahead; NaN: none yet). The three FP64 quotients
+        // per cell and direction bounded the FP64 passes of a mixed solve: 64³, S8, two groups
+        // 62.8 ms with them, 58.8 so.
+        R hx[RECIP ? DB : 1], hy[RECIP ? DB : 1], hz[RECIP ? DB : 1], dxc = R(NAN), dxn = R(0);
+        if constexpr (RECIP) {
+            dxn = P.dx[fx ? 0 : nx - 1];
+#pragma unroll
+            for (int k = 0; k < DB; k++) {
+                const bool in = pok && k < cnt;
+                hx[k] = R(0);
+                hy[k] = in ? oct_div(fabs(P.cosv[nd + first + k]), P.dy[iy]) : R(0);
+                hz[k] = in ? oct_div(fabs(P.cosv[2 * nd + first + k]), P.dz[iz]) : R(0);
+            }
+        }
         wait_up(0);
         __syncthreads();
         stage_cells(0);
@@ -502,21 +517,25 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                 const R S0 = mS[m], sq = mQ[m];
                 const R idx = xs_sm ? idxs[ix] : (R)(1.0 / P.dx[ix]);
                 if constexpr (RECIP) {
+                    if (dxn != dxc) {  // another width than the last cell's
+                        dxc = dxn;
+#pragma unroll
+                        for (int k = 0; k < DB; k++)
+                            if (k < cnt) hx[k] = oct_div(fabs(P.cosv[first + k]), dxc);
+                    }
+                    dxn = P.dx[ixx + 1 < nx ? (fx ? ix + 1 : ix - 1) : ix];
 #pragma unroll
                     for (int k = 0; k < DB; k++) {
                         if (k >= cnt) continue;
                         R d[6];
                         load6(d, dc + k * DC);
-                        const int n = first + k;
-                        const R hx = oct_div(fabs(P.cosv[n]), P.dx[ix]), hy = oct_div(fabs(P.cosv[nd + n]), P.dy[iy]);
-                        const R hz = oct_div(fabs(P.cosv[2 * nd + n]), P.dz[iz]);
                         R S = S0, q = v[k];
-                        S += hx * d[0];
-                        S += hy * d[1];
-                        S += hz * d[2];
-                        q += hx * (d[3] * fxs[k]);
-                        q += hy * (d[4] * fyi[k]);
-                        q += hz * (d[5] * fzi[k]);
+                        S += hx[k] * d[0];
+                        S += hy[k] * d[1];
+                        S += hz[k] * d[2];
+                        q += hx[k] * (d[3] * fxs[k]);
+                        q += hy[k] * (d[4] * fyi[k]);
+                        q += hz[k] * (d[5] * fzi[k]);
                         v[k] = q * oct_div(1.0, S);
                         fxs[k] = w1x * fxs[k] + gox * v[k];
                         fyi[k] = w1y * fyi[k] + goy * v[k];
@@ -655,7 +674,8 @@ __device__ __forceinline__ float recip(float s) { return __frcp_rn(s); }
 // works out its cells' coefficients (collision term, reciprocal, face factors: independent of the
 // faces) together, in registers, and a step is left with the shuffle and the cell's few dependent
 // operations. The piece's inputs come by cp.async two pieces ahead into the warp's own tile, 8 lanes
-// to a row's run of 8 cells; the outputs leave the same way.
+// to a row's run of 8 cells; the outputs leave the same way. 128×128, S12, FP64: 250 us (one load per
+// cell in flight, a barrier per step), 130 (8 loads ahead), 95 now.
 #define RB_2D_K 8
 // elements of a warp's tile of one array: 32 rows of K cells, padded to an odd stride
 #define RB_2D_TILE (32 * (RB_2D_K + 1))
@@ -825,7 +845,7 @@ __device__ __noinline__ void sweep2d_pf(Team &t, const DevProblem &P, GroupShare
 // the material and the widths only, so a lane keeps its inverse in registers along the row and
 // factors again where the material or a width changes; a cell is then a product with the inverse.
 // (The run-time shaped solve, which stays for the other shapes, eliminates every cell's matrix in
-// local memory: 9.4 us a step at 41×30, S6, four moments.)
+// local memory: 9.4 us a step at 41×30, S6, four moments; 0.9 here.)
 #define RB_2DHI_PF 4
 template <int NM, int NF, int NE, bool CSD>
 struct Sweep2dHi {
