@@ -23,6 +23,7 @@
 #pragma once
 #include <type_traits>
 
+#include "rb_quot.cuh"
 #include "rb_sweep_md.cuh"
 #include "rb_tc.cuh"
 
@@ -159,28 +160,6 @@ __device__ __forceinline__ bool wait_progress(const unsigned long long *f, unsig
     }
     return false;
 }
-
-// q / S of a cell. FP32 (mixed form): the fast reciprocal-based division, whose 2-ulp error the
-// FP64 defect correction absorbs. FP64 (plain form): the correctly rounded quotient by Newton's
-// reciprocal and Markstein's final correction (P. Markstein, "Computation of elementary functions
-// on the IBM RISC System/6000 processor", 1990) without a branch, so the chains of a cell's
-// directions interleave; the divide instruction sequence ends each one in a branch. Operands
-// outside the range where the correction is exact take the divide.
-__device__ __forceinline__ bool oct_div_range(double s) {
-    const double a = fabs(s);
-    return a > 1e-140 && a < 1e140;
-}
-__device__ __forceinline__ double oct_div_fast(double q, double s) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
-    r = fma(r, fma(-s, r, 1.0), r);
-    r = fma(r, fma(-s, r, 1.0), r);
-    const double v = q * r;
-    return fma(fma(-s, v, q), r, v);
-}
-__device__ __forceinline__ double oct_div(double q, double s) { return oct_div_range(s) ? oct_div_fast(q, s) : q / s; }
-__device__ __forceinline__ bool oct_div_range(float) { return true; }
-__device__ __forceinline__ float oct_div_fast(float q, float s) { return __fdividef(q, s); }
 
 // the six constants of a direction, as 16-byte loads
 __device__ __forceinline__ void load6(double (&d)[6], const double *p) {
@@ -452,8 +431,8 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
             for (int k = 0; k < DB; k++) {
                 const bool in = pok && k < cnt;
                 hx[k] = R(0);
-                hy[k] = in ? oct_div(fabs(P.cosv[nd + first + k]), P.dy[iy]) : R(0);
-                hz[k] = in ? oct_div(fabs(P.cosv[2 * nd + first + k]), P.dz[iz]) : R(0);
+                hy[k] = in ? quot(fabs(P.cosv[nd + first + k]), P.dy[iy]) : R(0);
+                hz[k] = in ? quot(fabs(P.cosv[2 * nd + first + k]), P.dz[iz]) : R(0);
             }
         }
         wait_up(0);
@@ -521,7 +500,7 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                         dxc = dxn;
 #pragma unroll
                         for (int k = 0; k < DB; k++)
-                            if (k < cnt) hx[k] = oct_div(fabs(P.cosv[first + k]), dxc);
+                            if (k < cnt) hx[k] = quot(fabs(P.cosv[first + k]), dxc);
                     }
                     dxn = P.dx[ixx + 1 < nx ? (fx ? ix + 1 : ix - 1) : ix];
 #pragma unroll
@@ -536,14 +515,15 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                         q += hx[k] * (d[3] * fxs[k]);
                         q += hy[k] * (d[4] * fyi[k]);
                         q += hz[k] * (d[5] * fzi[k]);
-                        v[k] = q * oct_div(1.0, S);
+                        v[k] = q * quot(1.0, S);
                         fxs[k] = w1x * fxs[k] + gox * v[k];
                         fyi[k] = w1y * fyi[k] + goy * v[k];
                         fzi[k] = w1z * fzi[k] + goz * v[k];
                     }
                 } else {
                     // every direction's collision term and right-hand side, then the quotients, then the
-                    // faces: three loops without a branch, so that the directions' chains overlap
+                    // faces: three loops without a branch, so that the directions' chains overlap.
+                    // FP32 takes the approximate division, whose 2-ulp error the FP64 defect correction absorbs.
                     R S[DB];
                     bool fast = true;
 #pragma unroll
@@ -554,11 +534,14 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
                         R q = v[k] + (d[3] * idx) * fxs[k] + (d[4] * idy) * fyi[k] + (d[5] * idz) * fzi[k];
                         if (CSD) q -= sq * fe[CSD ? k : 0];
                         v[k] = q;
-                        fast = fast && oct_div_range(S[k]);
+                        if constexpr (sizeof(R) == 8) fast &= (k >= cnt) | (quot_in(q) & quot_div_in(S[k]));
                     }
                     if (fast) {
 #pragma unroll
-                        for (int k = 0; k < DB; k++) v[k] = oct_div_fast(v[k], S[k]);
+                        for (int k = 0; k < DB; k++) {
+                            if constexpr (sizeof(R) == 8) v[k] = quot_by(v[k], S[k], quot_rcp(S[k]));
+                            else v[k] = __fdividef(v[k], S[k]);
+                        }
                     } else {
 #pragma unroll
                         for (int k = 0; k < DB; k++) v[k] = v[k] / S[k];
@@ -647,19 +630,6 @@ __device__ __forceinline__ void sweep3d_run(Team &t, const DevProblem &P, GroupS
     RB_OCT_RUN(OctDB<R>::value)
 #undef RB_OCT_RUN
 }
-
-// q / s given r = 1 / s correctly rounded: Markstein's correction of q·r, the correctly rounded
-// quotient. The reciprocal does not wait for the cell's faces, the two products do.
-__device__ __forceinline__ double div_by(double q, double s, double r) {
-    const double v = q * r;
-    return fma(fma(-s, v, q), r, v);
-}
-__device__ __forceinline__ float div_by(float q, float s, float r) {
-    const float v = q * r;
-    return fmaf(fmaf(-s, v, q), r, v);
-}
-__device__ __forceinline__ double recip(double s) { return oct_div(1.0, s); }
-__device__ __forceinline__ float recip(float s) { return __frcp_rn(s); }
 
 // 2D, one-moment cells: sweep_md's wavefront with the arithmetic in R (FP64 or FP32) over an
 // angular buffer held cells fastest.
@@ -792,7 +762,7 @@ __device__ __noinline__ void sweep2d_pf(Team &t, const DevProblem &P, GroupShare
                 double *e = es + (p & 1) * TS + lane * (K + 1);
                 const int *mm = ms + (p & 1) * TS + lane * (K + 1);
                 R cS[K], cr[K], cq[K], cax[K], cf[K], ce[CSD ? K : 1], cQ[CSD ? K : 1];
-                bool in[K];
+                bool in[K], far = false;
 #pragma unroll
                 for (int u = 0; u < K; u++) {
                     in[u] = row && (unsigned)(c0 + u) < (unsigned)nx;
@@ -810,21 +780,42 @@ __device__ __noinline__ void sweep2d_pf(Team &t, const DevProblem &P, GroupShare
                     }
                 }
 #pragma unroll
-                for (int u = 0; u < K; u++) cr[u] = recip(cS[u]);
-#pragma unroll
                 for (int u = 0; u < K; u++) {
-                    // X face of the row and Y face of the column (sn_sweep_2D.jl:71-132)
-                    const R up = __shfl_up_sync(0xffffffffu, Fy, 1);
-                    const R F1 = lane == 0 ? cf[u] : up;
-                    R qq = cq[u] + cax[u] * F0 + cay * F1;
-                    if (CSD) qq -= cQ[CSD ? u : 0] * ce[CSD ? u : 0];
-                    const R v = div_by(qq, cS[u], cr[u]);
-                    const R F0o = w1x * F0 + ox * v;
-                    Fy = w1y * F1 + oy * v;
-                    F0 = in[u] ? F0o : F0;
-                    q[u] = v;
-                    if (CSD && eou) e[u] = (double)(w1e * ce[CSD ? u : 0] + eout * v);
-                    if (keep && in[u]) yf[c0 + u] = Fy;
+                    cr[u] = quot_rcp(cS[u]);
+                    far |= in[u] & !quot_div_in(cS[u]);
+                }
+                // X face of the row and Y face of the column (sn_sweep_2D.jl:71-132); true where a dividend
+                // of the piece is outside quot_by's range
+                auto steps = [&](auto divide) {
+                    bool out = false;
+#pragma unroll
+                    for (int u = 0; u < K; u++) {
+                        const R up = __shfl_up_sync(0xffffffffu, Fy, 1);
+                        const R F1 = lane == 0 ? cf[u] : up;
+                        R qq = cq[u] + cax[u] * F0 + cay * F1;
+                        if (CSD) qq = fma(-cQ[CSD ? u : 0], ce[CSD ? u : 0], qq);
+                        R v;
+                        if constexpr (decltype(divide)::value) {
+                            v = qq / cS[u];
+                        } else {
+                            v = quot_by(qq, cS[u], cr[u]);
+                            out |= in[u] & !quot_in(qq);
+                        }
+                        const R F0o = w1x * F0 + ox * v;
+                        Fy = w1y * F1 + oy * v;
+                        F0 = in[u] ? F0o : F0;
+                        q[u] = v;
+                        if (CSD && eou) e[u] = (double)fma(w1e, ce[CSD ? u : 0], eout * v);
+                        if (keep && in[u]) yf[c0 + u] = Fy;
+                    }
+                    return out;
+                };
+                const R F0p = F0, Fyp = Fy;
+                far |= steps(std::false_type{});
+                if (__any_sync(0xffffffffu, far)) {  // the piece again, by divisions
+                    F0 = F0p;
+                    Fy = Fyp;
+                    steps(std::true_type{});
                 }
                 __syncwarp();
                 store(p);
