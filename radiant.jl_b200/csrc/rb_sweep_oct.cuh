@@ -53,7 +53,7 @@ __device__ __forceinline__ int oct_group(const DevProblem &P, int db, int g, int
 }
 
 // The problem is a one-moment 2D/3D problem (every closure of order 1).
-__device__ __forceinline__ bool one_moment_md(const DevProblem &P) {
+__host__ __device__ __forceinline__ bool one_moment_md(const DevProblem &P) {
     return P.nm5 == 1 && P.nmf[0] == 1 && P.nmf[1] == 1 && (P.ndims < 3 || P.nmf[2] == 1) && P.nm4 == 1;
 }
 
@@ -111,7 +111,7 @@ __host__ __device__ constexpr long long oct3d_smem(bool csd) { return Oct3dSmem<
 
 // Tile height in y: a power of two up to RB_OCT_TILE, so that a pencil's lower neighbour is the
 // previous lane of the same warp.
-__device__ __forceinline__ int oct_ty(int ny) {
+__host__ __device__ __forceinline__ int oct_ty(int ny) {
     int ty = 1;
     while (ty * 2 <= ny && ty * 2 <= RB_OCT_TILE) ty *= 2;
     return ty;
@@ -119,13 +119,21 @@ __device__ __forceinline__ int oct_ty(int ny) {
 
 // The 3D octant sweep applies: one-moment cells, one octant batch's tiles fit in the team, every
 // CTA of the team has a progress flag, and the step and round counts fit their bit fields.
-__device__ __forceinline__ bool oct3d_ok(const DevProblem &P, int ncta, long long smem_bytes, int mixed) {
+__host__ __device__ __forceinline__ bool oct3d_ok(const DevProblem &P, int ncta, long long smem_bytes, int mixed) {
     if (P.ndims != 3 || !one_moment_md(P) || ncta > RB_OCT_MAXCTA) return false;
-    if (P.nx + 2 * RB_OCT_TILE >= (1 << 20) || P.nd >= (1 << 12) || (long long)P.nd * P.ncell >= (1LL << 32)) return false;
-    const int TY = oct_ty(P.ny), TZ = min(P.nz, RB_OCT_TILE);
+    if (P.nx + 2 * RB_OCT_TILE >= (1 << 20) || P.nd >= (1 << 12)) return false;
+    const int TY = oct_ty(P.ny), TZ = P.nz < RB_OCT_TILE ? P.nz : RB_OCT_TILE;
     const int ntiles = ((P.ny + TY - 1) / TY) * ((P.nz + TZ - 1) / TZ);
     const long long need = mixed ? oct3d_smem<float>(P.csd) : oct3d_smem<double>(P.csd);
     return ntiles <= ncta && smem_bytes >= need;
+}
+
+// The angular arrays' offset of direction n at x column 0 (in sweep order) of pencil (qy, qz) of an
+// octant's sweep (fx, fy, fz: along the axis or against it); a column further is ±nd from there.
+// 64 bits: 2^32 values are 416×192×192 cells with the 288 directions of S16.
+__host__ __device__ __forceinline__ long long oct_offset(const DevProblem &P, bool fx, bool fy, bool fz, int qy, int qz, int n) {
+    const long long row = (fy ? qy : P.ny - 1 - qy) + (long long)P.ny * (fz ? qz : P.nz - 1 - qz);
+    return P.nd * (P.nx * row + (fx ? 0 : P.nx - 1)) + n;
 }
 
 // asynchronous global -> shared copies (cp.async, L1-allocating), and their groups
@@ -353,14 +361,14 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
             }
         };
         const R idy = pok ? (R)(1.0 / P.dy[iy]) : R(0), idz = pok ? (R)(1.0 / P.dz[iz]) : R(0);
-        const unsigned c0 = (unsigned)nx * (iy + ny * iz);  // the pencil's first cell
+        const long long c0 = (long long)nx * (iy + ny * iz);  // the pencil's first cell
         const int dstep = jy + jz;                          // the pencil's first step
         // element e = lane + 32·i of the warp's cells: part e % parts of pencil e / parts: its offset
         // in ψ at x column −(steps it runs behind), its steps behind, its place in a stage
         constexpr int NE = DB / VW;
-        unsigned eo[NE];
+        long long eo[NE];
         int ed[NE], ep[NE];
-        const unsigned estep = fx ? (unsigned)nd : 0u - (unsigned)nd;  // a column further
+        const long long estep = fx ? nd : -nd;  // a column further
 #pragma unroll
         for (int i = 0; i < NE; i++) {
             const int e = lane + 32 * i, pl = e / parts, part = e - pl * parts;
@@ -369,8 +377,7 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
             const bool ok = i < parts && pm < TY * TZ && qy < ny && qz < nz;
             ed[i] = ok ? py + pz : 1 << 28;
             ep[i] = pl * CS + part * VW;
-            const unsigned row = (unsigned)nx * ((fy ? qy : ny - 1 - qy) + ny * (fz ? qz : nz - 1 - qz));
-            eo[i] = ok ? (unsigned)nd * (row + (fx ? 0 : nx - 1)) + first + part * VW - (unsigned)ed[i] * estep : 0;
+            eo[i] = ok ? oct_offset(P, fx, fy, fz, qy, qz, first + part * VW) - ed[i] * estep : 0;
         }
         // the warp's cells of step s into stage s & 1
         auto stage_cells = [&](int s) {
@@ -378,7 +385,7 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
 #pragma unroll
             for (int i = 0; i < NE; i++) {
                 if (i < parts && (unsigned)(s - ed[i]) < (unsigned)nx) {
-                    const unsigned o = eo[i] + (unsigned)s * estep;
+                    const long long o = eo[i] + s * estep;
                     cp_async<VW * (int)sizeof(R)>(qb + st + ep[i], psi + o);
                     if (CSD && phiE_in) cp_async<VW * 8>(eb + st + ep[i], phiE_in + o);
                 }
@@ -389,7 +396,7 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
 #pragma unroll
             for (int i = 0; i < NE; i++) {
                 if (i < parts && (unsigned)(s - ed[i]) < (unsigned)nx) {
-                    const unsigned o = eo[i] + (unsigned)s * estep;
+                    const long long o = eo[i] + s * estep;
                     if constexpr (VW == 2) {
                         using R2 = typename Pair<R>::type;
                         *reinterpret_cast<R2 *>(psi + o) = *reinterpret_cast<const R2 *>(qb + st + ep[i]);
