@@ -737,8 +737,8 @@ int required(const rb_sn_problem *P, const Derived &D, Layout &L, size_t offs[64
     return k;
 }
 
-// Cluster size and shared memory of a launch (one CTA per SM): GroupShared plus, when some 1D
-// problem can take the local pass, a local region of all the shared memory left. The cluster:
+// Cluster size and shared memory of a launch (one CTA per SM): GroupShared plus a region of all the
+// shared memory left, for the local 1D pass, the 2D/3D sweeps and the products. The cluster:
 //   LAUNCH_FIXED   the caller's size;
 //   LAUNCH_SERVE   the caller's size, doubled (up to 4×) until the local pass fits;
 //   LAUNCH_BATCH   from 4 CTAs up, the smallest size that still gives no more teams than
@@ -800,8 +800,7 @@ int launch_solve(rb_context *ctx, DevProblem **list, int n, int *queue, int nsm,
                  const std::vector<const DevProblem *> &hs, int mode) {
     if (cluster < 1) cluster = 1;
     if (cluster > RB_MAXCLUSTER) cluster = RB_MAXCLUSTER;
-    const LaunchShape sh =
-        choose_shape((ctx && !ctx->local1d) ? std::vector<const DevProblem *>() : hs, cluster, mode, nsm);
+    const LaunchShape sh = choose_shape(hs, cluster, mode, nsm);
     cluster = sh.cluster;
     const size_t smem = sh.smem;
     const int local_bytes = (int)sh.local_bytes;
@@ -1025,6 +1024,7 @@ int place_problem(rb_context *ctx, const rb_sn_problem *P, const Derived &D, con
     h.psi_sc = P->ndims == 2 ? 1 : nd;
     h.pe_sn = P->ndims == 2 ? (long long)h.nm4 * D.ncell : 1;
     h.recip = mixed_recip(h, !D.tc_m2d.empty());
+    h.local1d = !ctx || ctx->local1d;
     h.noct = D.noct;
     for (int o = 0; o <= 8; o++) h.oct_start[o] = D.oct_start[o];
 #define DP(T, k) (reinterpret_cast<T *>(b + o[k]))

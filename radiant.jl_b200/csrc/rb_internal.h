@@ -34,6 +34,7 @@ struct DevProblem {
     long long nphi, nstate, off_b[3], nb[3];
     long long fcells[3];  // boundary face cells per axis
     int recip;         // mixed 3D form: the FP64 passes solve a cell by the reciprocal (rb_capi.cu)
+    int local1d;       // 1D: the local pass may be taken (0: RB_LOCAL1D=0)
     int noct;          // direction groups: 1 (1D), 4 quadrants (2D), 8 octants (3D)
     int oct_start[9];  // device directions of group o: [oct_start[o], oct_start[o+1]); 2D/3D
                        // problems hold their directions sorted by group (bit 0: μ < 0,

@@ -69,7 +69,7 @@ __host__ __device__ __forceinline__ long long local1d_op_bytes(const DevProblem 
 // whether a problem takes the local pass on a cluster of `ncta` CTAs with `local_bytes` of
 // shared memory beyond the per-CTA state
 __host__ __device__ __forceinline__ bool local1d_ok(const DevProblem &P, int ncta, long long local_bytes) {
-    return P.ndims == 1 && local1d_shape(P) && P.nd <= RB_THREADS && local1d_bytes(P, ncta, false) <= local_bytes;
+    return P.local1d && P.ndims == 1 && local1d_shape(P) && P.nd <= RB_THREADS && local1d_bytes(P, ncta, false) <= local_bytes;
 }
 // whether its Gram-Schmidt loop also keeps the slice of w in shared memory
 __host__ __device__ __forceinline__ bool local1d_w(const DevProblem &P, int ncta, long long local_bytes) {
