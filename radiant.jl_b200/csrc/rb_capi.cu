@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "../../include/radiant_b200.h"
+#include "rb_launch.cuh"
 #include "rb_solve.cuh"
 
 
@@ -737,17 +738,8 @@ int required(const rb_sn_problem *P, const Derived &D, Layout &L, size_t offs[64
     return k;
 }
 
-// Cluster size and shared memory of a launch (one CTA per SM): GroupShared plus a region of all the
-// shared memory left, for the local 1D pass, the 2D/3D sweeps and the products. The cluster:
-//   LAUNCH_FIXED   the caller's size;
-//   LAUNCH_SERVE   the caller's size, doubled (up to 4×) until the local pass fits;
-//   LAUNCH_BATCH   from 4 CTAs up, the smallest size that still gives no more teams than
-//                  problems (a large batch runs many small teams, a small one a few large
-//                  teams), among the sizes at which every 1D problem fits the local pass with its
-//                  Gram-Schmidt slice in shared memory (else, fits it at all). Below 4 CTAs a team
-//                  is slower per pass than the extra teams gain, measured on B200.
-// Problems that do not fit take the team-wide pass.
-enum { LAUNCH_FIXED = 0, LAUNCH_SERVE = 1, LAUNCH_BATCH = 2 };
+// Cluster size (rb_launch.cuh) and shared memory of a launch (one CTA per SM): GroupShared plus a
+// region of all the shared memory left, for the local 1D pass, the 2D/3D sweeps and the products.
 struct LaunchShape {
     int cluster;
     long long local_bytes;
@@ -762,35 +754,8 @@ static LaunchShape choose_shape(const std::vector<const DevProblem *> &hs, int c
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const long long gsz = (long long)sizeof(rb::GroupShared);
     const long long b1 = (std::min<long long>(optin, (long long)per_sm - reserved) - gsz) & ~15LL;
-    LaunchShape sh{cluster, 0, (size_t)gsz};
-    if (hs.empty() || b1 <= 0) return sh;
-    auto fits = [&](int C, bool w) {  // every local-shaped 1D problem fits the local pass at cluster C
-        for (const DevProblem *h : hs)
-            if (rb::local1d_ok(*h, C, 1LL << 40) && !(w ? rb::local1d_w(*h, C, b1) : rb::local1d_ok(*h, C, b1)))
-                return false;
-        return true;
-    };
-    int C = cluster;
-    if (mode == LAUNCH_SERVE) {
-        for (int c = cluster; c <= std::min(RB_MAXCLUSTER, 4 * cluster); c *= 2)
-            if (fits(c, false)) { C = c; break; }
-    } else if (mode == LAUNCH_BATCH) {
-        const int n = (int)hs.size();
-        for (int w = 1; w >= 0 && C == cluster; w--) {
-            int best = -1, largest = -1;
-            for (int c = 4; c <= RB_MAXCLUSTER; c *= 2) {
-                if (!fits(c, w != 0)) continue;
-                largest = c;
-                if (best < 0 && nsm / c <= n + n / 20) best = c;
-            }
-            if (best < 0) best = largest;
-            if (best > 0) { C = best; break; }
-        }
-    }
-    sh.cluster = C;
-    sh.local_bytes = b1;
-    sh.smem = (size_t)(gsz + b1);
-    return sh;
+    if (b1 <= 0) return {cluster, 0, (size_t)gsz};
+    return {choose_cluster(hs, cluster, mode, nsm, b1), b1, (size_t)(gsz + b1)};
 }
 
 // Launches the persistent solve kernel as clusters of `cluster` CTAs (one team per problem),
@@ -831,11 +796,11 @@ int launch_solve(rb_context *ctx, DevProblem **list, int n, int *queue, int nsm,
     return RB_OK;
 }
 
-// One 2D/3D problem on every SM: a cooperative launch of one CTA per SM (the team is the grid),
-// with the shared memory of the 3D octant sweep after GroupShared.
+// One 2D/3D problem on every SM: a cooperative launch of one CTA per SM (the team is the grid).
 int launch_grid(rb_context *ctx, DevProblem *prob, const DevProblem &hp, cudaStream_t s) {
-    // the region after GroupShared serves the 3D octant sweep and the tensor-core products; it is
-    // sized to what this problem uses, since the rest of the SM's 256 KB stays L1 cache
+    // the region after GroupShared serves, one after another, the 2D/3D sweeps, the tensor-core and
+    // FP64 products, the boundary products and BiCGStab's streamed loops; it is sized to what this
+    // problem uses, since the rest of the SM's 256 KB stays L1 cache
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     const long long avail = (optin - (long long)sizeof(rb::GroupShared)) & ~1023LL;

@@ -1,4 +1,5 @@
-"""Which 3D problems the octant sweep takes, and its offsets into the angular arrays, on the host."""
+"""Which 3D problems the octant sweep takes, its offsets into the angular arrays, and the team size of a
+launch, on the host."""
 import ctypes
 import os
 import subprocess
@@ -37,3 +38,18 @@ def test_octant_offsets(lib, ns, nd):
             iy, iz = qy if f & 2 else ny - 1 - qy, qz if f & 4 else nz - 1 - qz
             ix = 0 if f & 1 else nx - 1
             assert lib.plan_oct_offset(nx, ny, nz, nd, f, qy, qz, n) == nd * (ix + nx * (iy + ny * iz)) + n
+
+
+FIXED, SERVE, BATCH = 0, 1, 2
+
+
+@pytest.mark.parametrize("n", [1, 24, 100])
+def test_team_size(lib, n):
+    # third-order energy closures have no local pass: such slabs keep the caller's size
+    for mode in (FIXED, SERVE, BATCH):
+        for cluster in (1, 4):
+            assert lib.plan_cluster(1, 3, 1, n, cluster, mode) == cluster
+    # slabs of the local pass and 2D problems: as many teams as problems, from 4 CTAs up
+    want = {1: 16, 24: 8, 100: 4}[n]
+    assert lib.plan_cluster(1, 1, 0, n, 4, BATCH) == lib.plan_cluster(2, 1, 0, n, 4, BATCH) == want
+    assert lib.plan_cluster(1, 1, 0, n, 2, FIXED) == lib.plan_cluster(2, 1, 0, n, 2, FIXED) == 2
