@@ -43,7 +43,8 @@ struct Prod64 {
     double *out;          // [i·so + col·ldo]
     long long so, ldo;
     // half of the directions only: those n whose (sel[n] >= 0) is selpos. selk: n is k (the others'
-    // operator columns are zero); else n is i (the others' outputs are left alone). null: all.
+    // operator columns and values of X are taken as zero, whatever X holds there); else n is i (the
+    // others' outputs are left alone). null: all.
     const double *sel = nullptr;
     bool selk = false, selpos = false;
     // both parts on a piece of k before the next piece (the columns are loaded once, not twice): the
@@ -82,6 +83,12 @@ __device__ __forceinline__ double lds64(uint32_t a) {
     return v;
 }
 
+__device__ __forceinline__ int lds32(uint32_t a) {
+    int v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+
 // asynchronous copy global -> shared of B bytes, zeros instead where `in` is false
 template <int B>
 __device__ __forceinline__ void cp_zfill(double *dst, const double *src, bool in) {
@@ -91,7 +98,8 @@ __device__ __forceinline__ void cp_zfill(double *dst, const double *src, bool in
 }
 
 // Rows [i0, i0 + 8·nt) of the operator into shared memory, zero beyond ni and nk: every copy in
-// flight at once (a row per warp, 16 bytes a lane where the operator's rows are aligned).
+// flight at once (a row per warp, 16 bytes a lane where the operator's rows are aligned). selk: the
+// first word of a row's padding says whether its k is in.
 __device__ __forceinline__ void prod_load_op(const Prod64 &a, double *op, int i0, int nt) {
     const int kp = prod_kp(a.nk), ld = 8 * nt + 4, parts = a.B ? 2 : 1;
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -102,6 +110,7 @@ __device__ __forceinline__ void prod_load_op(const Prod64 &a, double *op, int i0
         const int k = pb ? r - kp : r;
         const double *src = (pb ? a.B : a.A) + (k < a.nk ? (long long)a.lda * k : 0);
         const bool kin = k < a.nk && !(a.sel && a.selk && (a.sel[k] >= 0.0) != a.selpos);
+        if (a.selk && lane == 0) *reinterpret_cast<int *>(op + r * ld + 8 * nt) = kin;
         if (vec) {
             for (int i = 2 * lane; i < 8 * nt; i += 64) {
                 const bool in = kin && i0 + i < a.ni;
@@ -119,7 +128,8 @@ __device__ __forceinline__ void prod_load_op(const Prod64 &a, double *op, int i0
 }
 
 // The column tiles w0, w0 + wstep, … (groups of MT tiles of 8) against the resident operator block.
-template <int NT, int MT>
+// SELK: a.selk (the test of k in the other products cost 128×128, S12 4 %).
+template <int NT, int MT, bool SELK>
 __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int i0, int w0, int wstep) {
     const Prod64 a = a_;
     const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
@@ -135,7 +145,7 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
     const uint32_t ob = (uint32_t)__cvta_generic_to_shared(op) + (uint32_t)(q * LD + r) * 8;
     const long long ngrp = (a.ncol + 8 * MT - 1) / (8 * MT);
     if (w0 >= ngrp) return;
-    const bool rows = a.sel && !a.selk;
+    const bool rows = a.sel && !SELK;
     const bool vec = !rows && a.so == 1 && (a.ldo % 2 == 0) && (reinterpret_cast<uintptr_t>(a.out) % 16 == 0) &&
                      (reinterpret_cast<uintptr_t>(a.pre) % 16 == 0);
     double xn[MT][CH];
@@ -193,6 +203,11 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
 #pragma unroll
                     for (int mt = 0; mt < MT; mt++) av[mt] = sc[mt][u] * xc[mt][u];
                     const uint32_t o = ob + (uint32_t)(ks * 4 + (pb ? kp : 0)) * (LD * 8);
+                    if constexpr (SELK) {
+                        const bool in = lds32(o + (uint32_t)(8 * NT - r) * 8) != 0;
+#pragma unroll
+                        for (int mt = 0; mt < MT; mt++) av[mt] = in ? av[mt] : 0.0;
+                    }
 #pragma unroll
                     for (int n = 0; n < NT; n++) {
                         const double b = lds64(o + n * 64);
@@ -257,10 +272,15 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
 // where every warp still gets one.
 __device__ __forceinline__ void prod_run(const Prod64 &a, const double *op, int i0, int nt, int w0, int wstep) {
     const bool pair = a.ncol >= 16LL * wstep;
-#define RB_PROD_CASE(NT_)                                       \
-    case NT_:                                                   \
-        if (pair) prod_tiles<NT_, 2>(a, op, i0, w0, wstep);     \
-        else prod_tiles<NT_, 1>(a, op, i0, w0, wstep);          \
+#define RB_PROD_CASE(NT_)                                                  \
+    case NT_:                                                              \
+        if (a.selk) {                                                      \
+            if (pair) prod_tiles<NT_, 2, true>(a, op, i0, w0, wstep);      \
+            else prod_tiles<NT_, 1, true>(a, op, i0, w0, wstep);           \
+        } else {                                                           \
+            if (pair) prod_tiles<NT_, 2, false>(a, op, i0, w0, wstep);     \
+            else prod_tiles<NT_, 1, false>(a, op, i0, w0, wstep);          \
+        }                                                                  \
         break;
     switch (nt) {
         RB_PROD_CASE(2)
