@@ -128,9 +128,14 @@ __device__ __forceinline__ void prod_load_op(const Prod64 &a, double *op, int i0
 }
 
 // The column tiles w0, w0 + wstep, … (groups of MT tiles of 8) against the resident operator block.
-// SELK: a.selk (the test of k in the other products cost 128×128, S12 4 %).
+// With a.selk a column in which the directions left out hold an infinity or NaN comes out non-finite (zero
+// operator columns times it): such a group is not stored, and the result is true; prod_run then calls the
+// SELK variant, which takes those directions' values as zero by the flags of the operator's rows. A look at
+// the sums is thus all that ordinary columns pay (the flags in every product: 128×128, S12 4 %; in the
+// boundary products alone, whose code then is not the M2D and D2M products': 41×30, S6, four moments and
+// 48×41×35, S8 electrons 2 %; a call of the SELK variant from here: 128×128, S12 11 %, by its registers).
 template <int NT, int MT, bool SELK>
-__device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int i0, int w0, int wstep) {
+__device__ __noinline__ bool prod_tiles(const Prod64 &a_, const double *op, int i0, int w0, int wstep) {
     const Prod64 a = a_;
     const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
     constexpr int LD = 8 * NT + 4;
@@ -144,8 +149,9 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
     const int nch = two && !inter ? 2 * npc : npc;
     const uint32_t ob = (uint32_t)__cvta_generic_to_shared(op) + (uint32_t)(q * LD + r) * 8;
     const long long ngrp = (a.ncol + 8 * MT - 1) / (8 * MT);
-    if (w0 >= ngrp) return;
-    const bool rows = a.sel && !SELK;
+    if (w0 >= ngrp) return false;
+    bool bad = false;
+    const bool rows = a.sel && !a.selk;
     const bool vec = !rows && a.so == 1 && (a.ldo % 2 == 0) && (reinterpret_cast<uintptr_t>(a.out) % 16 == 0) &&
                      (reinterpret_cast<uintptr_t>(a.pre) % 16 == 0);
     double xn[MT][CH];
@@ -227,6 +233,19 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
                 }
             }
         }
+        if (!SELK && a.selk) {
+            int most = 0;
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                for (int n = 0; n < NT; n++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) most = max(most, __double2hiint(acc[mt][n][e]) & 0x7fffffff);
+            if (__any_sync(0xffffffffu, most >= 0x7ff00000)) {
+                bad = true;
+                continue;
+            }
+        }
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
             const long long col = (g * MT + mt) * 8 + r;
@@ -266,20 +285,22 @@ __device__ __noinline__ void prod_tiles(const Prod64 &a_, const double *op, int 
             }
         }
     }
+    return bad;
 }
 
 // Dispatch on the row tiles of the block; pairs of column tiles per warp (half the operator reads)
-// where every warp still gets one.
+// where every warp still gets one. Sums added to the outputs of earlier ones (a cut along k) cannot be
+// computed twice and take the flags at once.
 __device__ __forceinline__ void prod_run(const Prod64 &a, const double *op, int i0, int nt, int w0, int wstep) {
-    const bool pair = a.ncol >= 16LL * wstep;
+    const bool pair = a.ncol >= 16LL * wstep, flags = a.selk && a.pre == a.out;
 #define RB_PROD_CASE(NT_)                                                  \
     case NT_:                                                              \
-        if (a.selk) {                                                      \
-            if (pair) prod_tiles<NT_, 2, true>(a, op, i0, w0, wstep);      \
-            else prod_tiles<NT_, 1, true>(a, op, i0, w0, wstep);           \
+        if (pair) {                                                        \
+            if (flags || prod_tiles<NT_, 2, false>(a, op, i0, w0, wstep))  \
+                prod_tiles<NT_, 2, true>(a, op, i0, w0, wstep);            \
         } else {                                                           \
-            if (pair) prod_tiles<NT_, 2, false>(a, op, i0, w0, wstep);     \
-            else prod_tiles<NT_, 1, false>(a, op, i0, w0, wstep);          \
+            if (flags || prod_tiles<NT_, 1, false>(a, op, i0, w0, wstep))  \
+                prod_tiles<NT_, 1, true>(a, op, i0, w0, wstep);            \
         }                                                                  \
         break;
     switch (nt) {
