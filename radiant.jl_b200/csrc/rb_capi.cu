@@ -941,7 +941,8 @@ ProblemRec *find(rb_context *ctx, rb_handle h) {
 // the octant sweep: the form those passes have had for the problems without CSD whose operators'
 // shared memory left no room for the octant sweep's FP64 stages (128 208 bytes). The FP32 passes
 // between them follow the last bit of these passes (BiCGStab carries it to 1e-8 of the flux), so the
-// form is part of the mixed result and stays.
+// form is part of the mixed result and stays. Cluster teams, which hold all of an SM's shared memory,
+// take the octant sweep's quotient there.
 static int mixed_recip(const DevProblem &h, bool tc) {
     if (h.precision != 1 || h.ndims != 3 || h.nm5 != 1 || h.csd) return 0;
     const long long avail = 183296;

@@ -131,11 +131,6 @@ struct Local1D {
     }
 };
 
-// state element of element j of the CTA's slice of a Krylov vector
-__device__ __forceinline__ long long local1d_elem(const Local1D &L, int j) {
-    return j < L.l1 ? L.e0 + j : L.eb + (j - L.l1);
-}
-
 // the FP64 operators into the region, once per problem
 __device__ __forceinline__ void local1d_load_ops(const DevProblem &P, Local1D &L) {
     if (!L.opM) return;

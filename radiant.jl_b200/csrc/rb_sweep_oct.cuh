@@ -17,9 +17,10 @@
 // Each cell sees the same upwind faces as in the reference's lexicographic order
 // (sn_sweep_3D.jl:73-110), so the result equals it up to rounding.
 //
-// 2D: the KBA wavefront of sweep_md (rows of a direction skewed by one column per row, y faces
-// handed between rows through shared memory), one direction per thread, with the cells' inputs
-// loaded several steps ahead.
+// 2D: the KBA wavefront of sweep_md (rows of a direction skewed by one column per row), a warp on 32
+// rows of a direction: y faces go from row to row by shuffle and from warp to warp through shared
+// memory, and the cells come by cp.async some steps ahead (sweep2d_pf, and sweep2d_hi for cells of
+// several moments).
 #pragma once
 #include <type_traits>
 
@@ -200,8 +201,9 @@ template <> struct Pair<double> { using type = double2; };
 // faces, cells, barrier. A lane that reads its own cell's directions touches a line per lane and
 // load, so a warp's 32 cells are staged together, cnt / VW neighbouring lanes on the run of one
 // cell, with each lane's pencils and offsets worked out once per task; the same lanes write the
-// results back. VW = 2: the batch's directions start and count even (pairs). Sweep at 64³, S8,
-// mixed: 2070 us (element-wise staging, addresses per element), 1030 (each thread its own cell), 960 now.
+// results back. VW = 2: the batch's directions start and count even (pairs). Sweep at 64³, S8, mixed,
+// mean of a solve's passes: 2070 us (element-wise staging, addresses per element), 1030 (staged by warps),
+// 810 now (faces leaving coalesced, |Ω|/Δ per pencil; FP32 passes 670, FP64 ones 1310).
 // RECIP: the cell as sweep_3d_tiles solves it (DevProblem::recip).
 template <typename R, int DB, int VW, bool CSD, bool RECIP, class Team>
 __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShared &gs, void *smem,
@@ -292,7 +294,7 @@ __device__ __noinline__ void sweep3d_oct(Team &t, const DevProblem &P, GroupShar
         // the last pencils of the tile, whose faces leave it
         const int jyE = min(TY, ny - tyq * TY) - 1, jzE = min(TZ, nz - tzq * TZ) - 1;
         // The faces entering the tile in a step, one direction of one pencil per item: pencils
-        // (0, j) for y faces, then (j, 0) for z faces; a thread has up to RB_OCT_ITEMS of them.
+        // (0, j) for y faces, then (j, 0) for z faces; a thread has up to NI of them.
         constexpr int NI = (2 * TT * DB + TP - 1) / TP;
         const double *isrc[NI];  // the item's face at x column 0
         double *iout[NI];        // and the same item's face leaving the tile, from its last pencils
