@@ -49,7 +49,7 @@ METRIC = "cell-dir-group updates/s"
 # proportion to the updates, so a launch's traffic is this times its updates:
 #   solve_local1d_kernel, 18 electron solves of the 1D batch reduced to 8 groups, FP64;
 #   solve_grid_kernel, the 3D photon problem reduced to one group, mixed and FP64 forms.
-TRAFFIC_BYTES_PER_UPDATE = {("c2", "fp64"): 399.8, ("c4", "mixed"): 140.9, ("c4", "fp64"): 158.2}
+TRAFFIC_BYTES_PER_UPDATE = {("c2", "fp64"): 407.4, ("c4", "mixed"): 119.6, ("c4", "fp64"): 140.2}
 PEAKS_PATH = os.path.join(ROOT, "MEASURED_PEAKS.json")
 
 
